@@ -66,7 +66,8 @@ def listed():
         # as the setup server does with the requests it holds.
         {"name": "hierarchies_24", "kind": "hierarchies", "count": 24, "specs": 3,
          "nmin": 1000, "nmax": 200000, "coarse": "f64"},
-        # One batch of uneven products with new patterns: plan and execute.
+        # One batch of uneven products, as a program with new patterns runs
+        # it: the batch is made, planned and executed.
         {"name": "batch_run_20", "kind": "batch_run", "count": 20, "specs": 7,
          "nmin": 1000, "nmax": 200000},
         # The numeric re-setup of a planned batch: patterns kept, values read anew.
@@ -206,9 +207,13 @@ class _Owned:
     def __init__(self, *objects):
         self.objects = objects
 
-    def __del__(self):
+    def free(self):
         for o in self.objects:
             o.free()
+        self.objects = ()
+
+    def __del__(self):
+        self.free()
 
 
 class _Memory:
@@ -259,13 +264,14 @@ def prepare(case, seed):
         As = [ctx.upload(_diffusion(d, 1000 * seed + i)) for i, d in enumerate(dims)]
         return _State(case, ctx=ctx, stream=stream, As=As, dims=dims, owner=_Owned(*As))
     products = [tuple(_galerkin(ctx, d, 1000 * seed + i, S.F64)) for i, d in enumerate(dims)]
+    owner = _Owned(*[m for p in products for m in p])
+    if kind == "batch_run":
+        return _State(case, ctx=ctx, products=products, owner=owner)
     batch = ctx.batch(products)
-    owner = _Owned(batch, *[m for p in products for m in p])
-    state = _State(case, ctx=ctx, batch=batch, owner=owner)
-    if kind == "batch_replay":
-        batch.plan()
-        state.out = [_arrays(batch.result(i), owner) for i in range(len(batch))]
-    return state
+    batch.plan()
+    owner = _Owned(batch, owner)
+    return _State(case, ctx=ctx, batch=batch, owner=owner,
+                  out=[_arrays(batch.result(i), owner) for i in range(len(batch))])
 
 
 def _galerkin(ctx, dims, seed, vt):
@@ -294,8 +300,10 @@ def run(state):
         owner = _Owned(*hs)
         return _packed([_levels(h, owner) for h in hs], state.stream)
     if kind == "batch_run":
-        state.batch.run()
-        return [_arrays(state.batch.result(i), state.owner) for i in range(len(state.batch))]
+        batch = state.ctx.batch(state.products)
+        owner = _Owned(batch)
+        batch.run()
+        return [_arrays(batch.result(i), owner) for i in range(len(batch))]
     if kind == "batch_replay":
         state.batch.execute()
         return state.out

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <cstdarg>
 #include <cstdio>
@@ -319,6 +320,32 @@ struct RowRunner {
                 return SP3MM_OK;
             }
         }
+        if (!direct && ctx->tune_G == 0 && G == 32 && p.retry_rows && b_max >= 0) {
+            if (pair_lanes_row_bytes(mode, 2 * p.S1) <= kLanesMaxWarpBytes) p.S1 *= 2;
+            const size_t per_warp = pair_lanes_row_bytes(mode, p.S1);
+            int warps = static_cast<int>(ctx->smem_budget / per_warp);
+            if (warps > 8) warps = 8;
+            if (warps >= 1) {
+                RowGeom geo{};
+                geo.G = 32;
+                geo.block = 32 * warps;
+                geo.smem = per_warp * warps;
+                const long long grid = (p.nrows + warps - 1) / warps;
+                const long long cap = static_cast<long long>(ctx->num_sms) * 16;
+                geo.grid = static_cast<int>(grid < cap ? grid : cap);
+                p.gtab = nullptr;
+                p.lg1 = lanes_layout(b_max, pa.B);
+                static const char* const kLanes[3] = {"pair.lanes.symb", "pair.lanes.num",
+                                                      "pair.lanes.book"};
+                cudaError_t e = cudaSuccess;
+                prof(ctx, kLanes[mode],
+                     [&] { e = launch_pair_lanes(pa, p, mode, geo, ctx->stream); });
+                if (e != cudaSuccess)
+                    return set_error(ctx, SP3MM_ECUDA, "lanes row kernel launch failed: %s",
+                                     cudaGetErrorString(e));
+                return SP3MM_OK;
+            }
+        }
         const size_t per_group = row_table_bytes(direct, mode, G, p.S1, p.S2);
         const int gpw = 32 / G;
         int warps = static_cast<int>(ctx->smem_budget / (per_group * gpw));
@@ -421,6 +448,55 @@ struct RowRunner {
         return SP3MM_OK;
     }
 };
+
+bool plain_tuning(const sp3mm_ctx* ctx) {
+    return ctx->tune_G == 0 && ctx->tune_d1 < 0 && ctx->tune_d2 < 0;
+}
+
+// Products whose longest rows bound every row's products by kBoundedProducts
+// need no bounds pass and no binning: the bound sizes one launch over all
+// rows (a bounds launch, two binning launches and a host round trip fewer:
+// the 64x64 product 106 -> 85 us).
+constexpr int kBoundedProducts = 512;
+// Of these, products of at least kReplayMinRows rows with bounds of at least
+// kReplayMinProducts try the replayed rows (rowreplay.cuh) first.  Below that
+// many rows its templates serve too few (direct, 7-point box: 6,840 rows 87 us
+// against 57 on the lanes kernel alone, 21,000 rows 126 against 127, 262,144
+// rows 0.95 ms against 1.51); with fewer products a row is one batch of the
+// lanes kernel, and the rows of A*P alternate between patterns.
+constexpr int kReplayMinRows = 16384;
+constexpr int kReplayMinProducts = 48;
+// A CTA's rows share one template: as many as the resident CTAs leave, at
+// least this many (128 rows: 60 % slower at 50,000 rows of a 5-point grid).
+constexpr int kReplayCtaRows = 32;
+constexpr int kReplayWarps = 4;         // per CTA
+constexpr int kReplayCtasPerSm = 5;     // by registers
+
+// Whether rows of at most k1 steps of l1 products (and, direct, of P rows of
+// at most l2) are bounded so, and the replayed kernel's capacities: columns
+// and stage-2 products are optimistic (7-point R*A rows: 224 products, 79
+// columns, 316 stage-2 products; a template that does not fit leaves its rows
+// to the lanes kernel).
+bool bounded_rows(bool direct, int k1, int l1, int n1, int l2, int n2, ReplayCaps* c) {
+    if (k1 < 0 || l1 < 0 || l2 < 0 || k1 > kReplayMaxColumns) return false;
+    const long long np = static_cast<long long>(k1) * l1;
+    if (np > kBoundedProducts) return false;
+    auto columns = [](int p, int n) {
+        const int c = p <= 96 ? p : std::max(96, p / 2);
+        return std::max(1, std::min({c, n, kReplayMaxColumns}));
+    };
+    c->np1 = std::max(4, static_cast<int>(np + 3) / 4 * 4);
+    c->k1 = std::max(1, k1);
+    c->ns1 = columns(c->np1, n1);
+    c->np2 = c->ns2 = 0;
+    if (direct) {
+        const long long np2 =
+            std::min<long long>(static_cast<long long>(c->ns1) * l2, c->np1 * 3 / 2);
+        c->np2 = std::max(4, static_cast<int>(np2 + 3) / 4 * 4);
+        c->ns2 = std::max(1, std::min(c->ns1 <= 64 ? c->ns1 : std::max(64, c->ns1 / 2), n2));
+    }
+    return true;
+}
 
 int finish_matrix(sp3mm_dcsr* C, DevBuf& rp, DevBuf& ci, DevBuf& v) {
     C->row_ptr = static_cast<int*>(rp.detach());
@@ -667,6 +743,151 @@ int product_rows(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, int o
     return finish_matrix(C, rp, ci, v);
 }
 
+// A product of bounded rows (bounded_rows): the replayed kernel over all rows
+// where it may pay, the lanes kernel over what it leaves, or over all rows.
+int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, int out_vt,
+                    const ReplayCaps& caps, long long s1_max, long long s2_max,
+                    unsigned long long out_bound, sp3mm_dcsr* C) {
+    const cudaStream_t st = ctx->stream;
+    DevBuf row_cnt, rp, ci, v, cnt_buf, retry, ub_ci, ub_v, row_off;
+    TRY(row_cnt.alloc(ctx, sizeof(int) * (static_cast<size_t>(M) + 1)));
+    TRY(cnt_buf.alloc(ctx, sizeof(Counters)));
+    TRY(retry.alloc(ctx, sizeof(int) * (static_cast<size_t>(M) + 1)));
+    Counters* dc = cnt_buf.as<Counters>();
+    CK(ctx, cudaMemsetAsync(dc, 0, sizeof(Counters), st));
+    RowParams p{};
+    p.nrows = M;
+    p.row_cnt = row_cnt.as<int>();
+    p.retry_rows = retry.as<int>();
+    p.retry_count = &dc->retry_count;
+    p.err = ctx->d_err;
+    p.c_vt = out_vt;
+    const bool replay = M >= kReplayMinRows && caps.np1 >= kReplayMinProducts;
+    DevBuf left;
+    if (replay) TRY(left.alloc(ctx, sizeof(int) * (static_cast<size_t>(M) + 1)));
+    int* n_left = left.as<int>() + M;
+    auto geometry = [&](int mode) {
+        RowGeom geo{};
+        geo.block = 32 * kReplayWarps;
+        geo.smem = replay_bytes(mode, caps, kReplayWarps);
+        const long long per_sm = std::max<long long>(
+            1, std::min<long long>(kReplayCtasPerSm, ctx->smem_optin / (geo.smem + 1024)));
+        geo.grid = static_cast<int>(std::min<long long>(
+            (M + kReplayCtaRows - 1) / kReplayCtaRows, per_sm * ctx->num_sms));
+        return geo;
+    };
+    // First table of the lanes kernel: the optimistic size of a row at the
+    // bound (launch_direct_bounds).
+    const int N1 = rr.direct ? rr.da.A.N : N;
+    long long need = std::min<long long>(
+        caps.np1 >> 2, static_cast<long long>(std::ceil(8.0 * std::sqrt(caps.np1 * 1.0))));
+    if (caps.np1 >= N1) need = N1;
+    auto rows = [&](int mode) -> int {
+        rr.mode = mode;
+        RowParams q = p;
+        if (replay) {
+            CK(ctx, cudaMemsetAsync(n_left, 0, sizeof(int), st));
+            const RowGeom geo = geometry(mode);
+            static const char* const kLabels[2][3] = {
+                {"pair.replay.symb", "pair.replay.num", "pair.replay.book"},
+                {"direct.replay.symb", "direct.replay.num", "direct.replay.book"}};
+            q.rcaps = caps;
+            q.left_rows = left.as<int>();
+            q.left_count = n_left;
+            cudaError_t e = cudaSuccess;
+            prof(ctx, kLabels[rr.direct ? 1 : 0][mode], [&] {
+                e = rr.direct ? launch_direct_replay(rr.da, q, mode, geo, st)
+                              : launch_pair_replay(rr.pa, q, mode, geo, st);
+            });
+            if (e != cudaSuccess)
+                return set_error(ctx, SP3MM_ECUDA, "replayed row kernel launch failed: %s",
+                                 cudaGetErrorString(e));
+            q.rows = left.as<int>();
+            q.nrows_dev = n_left;
+        }
+        q.S1 = slots_for_need(std::max<long long>(1, need), 32);
+        q.S2 = rr.direct ? q.S1 : 0;
+        DevBuf gtab;
+        return rr.launch(q, 32, gtab);
+    };
+    TailReads tr{};
+    if (flavour == SP3MM_SYMBNUM) {
+        TRY(rows(kSymb));
+        TRY(scan_read(ctx, M, row_cnt.as<int>(), rp, &dc->retry_count, &tr));
+        if (tr.err) return check_device_err(ctx);
+        if (tr.retry > 0) {
+            TRY(rr.run_retry(p, tr.retry, retry, s1_max, s2_max));
+            TRY(scan_read(ctx, M, row_cnt.as<int>(), rp, nullptr, &tr));
+            if (tr.err) return check_device_err(ctx);
+        }
+    } else {
+        const size_t eb = sizeof(int) + vbytes(out_vt);
+        unsigned long long cap = std::min<unsigned long long>(
+            out_bound,
+            std::max<unsigned long long>(1ULL << 20,
+                                         8ULL * static_cast<unsigned long long>(rr.operand_nnz())));
+        if (cap * eb > (size_t(1) << 30) && pool_idle_bytes(ctx) < cap * eb)
+            cap = std::min<unsigned long long>(
+                cap, std::max<unsigned long long>(1ULL << 20, free_device_bytes(ctx) / 2 / eb));
+        if (replay)   // every warp may leave most of its last handout unused
+            cap += static_cast<unsigned long long>(geometry(kNumBook).grid) * kReplayWarps *
+                   kReplayBook;
+        TRY(ub_ci.alloc(ctx, sizeof(int) * cap));
+        TRY(ub_v.alloc(ctx, vbytes(out_vt) * cap));
+        TRY(row_off.alloc(ctx, sizeof(long long) * (static_cast<size_t>(M) + 1)));
+        p.cursor = &dc->cursor;
+        p.cap = cap;
+        p.row_off = row_off.as<long long>();
+        p.ub_ci = ub_ci.as<int>();
+        p.ub_v = ub_v.p;
+        TRY(rows(kNumBook));
+        TRY(scan_read(ctx, M, row_cnt.as<int>(), rp, &dc->retry_count, &tr));
+        for (int pass = 0; pass < 2; ++pass) {
+            if (tr.err & ~kErrBook) return check_device_err(ctx);
+            if (tr.err == kErrBook) {
+                CK(ctx, cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), st));
+                ub_ci.release();
+                ub_v.release();
+                return product_bounded(ctx, rr, M, N, SP3MM_SYMBNUM, out_vt, caps, s1_max, s2_max,
+                                       out_bound, C);
+            }
+            if (pass == 1 || tr.retry <= 0) break;
+            TRY(rr.run_retry(p, tr.retry, retry, s1_max, s2_max));
+            TRY(scan_read(ctx, M, row_cnt.as<int>(), rp, nullptr, &tr));
+        }
+    }
+    const long long nnz = tr.total;
+    const int cmax = tr.max_row;
+    if (nnz < 0 || nnz >= INT32_MAX)
+        return set_error(ctx, SP3MM_ELIMIT, "result has too many nonzeros");
+    TRY(ci.alloc(ctx, sizeof(int) * static_cast<size_t>(nnz)));
+    TRY(v.alloc(ctx, vbytes(out_vt) * static_cast<size_t>(nnz)));
+    if (flavour == SP3MM_SYMBNUM) {
+        p.c_rp = rp.as<int>();
+        p.c_ci = ci.as<int>();
+        p.c_v = v.p;
+        CK(ctx, cudaMemsetAsync(&dc->retry_count, 0, sizeof(int), st));
+        TRY(rows(kNumExact));
+        TRY(read_retry_err(ctx, &dc->retry_count, &tr));
+        if (tr.retry > 0 && !tr.err) {
+            TRY(rr.run_retry(p, tr.retry, retry, s1_max, s2_max));
+            TRY(read_retry_err(ctx, nullptr, &tr));
+        }
+        if (tr.err) return check_device_err(ctx);
+    } else {
+        prof(ctx, "compact", [&] {
+            launch_compact(M, row_cnt.as<int>(), row_off.as<long long>(), ub_ci.as<int>(), ub_v.p,
+                           rp.as<int>(), ci.as<int>(), v.p, out_vt, st);
+        });
+    }
+    C->M = M;
+    C->N = N;
+    C->nnz = nnz;
+    C->val_type = out_vt;
+    C->max_row = cmax;
+    return finish_matrix(C, rp, ci, v);
+}
+
 // ---------------------------------------------------------------------------
 // C = A*B.
 int spmm_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flavour, int out_vt,
@@ -683,6 +904,14 @@ int spmm_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flav
     const double products = (A.M ? static_cast<double>(A.nnz) / A.M : 0.0) *
                             (B.M ? static_cast<double>(B.nnz) / B.M : 0.0);
     if (ctx->tune_G == 0 && products <= 8.0) G = 4;
+    ReplayCaps caps;
+    if (G == 32 && plain_tuning(ctx) &&
+        bounded_rows(false, A.max_row, B.max_row, B.N, 0, 0, &caps)) {
+        RowRunner rr{ctx, false, kSymb, {}, PairRowArgs{view(A), view(B)}, -1, B.max_row};
+        return product_bounded(ctx, rr, M, B.N, flavour, out_vt, caps,
+                               std::min<long long>(caps.np1, B.N), 0,
+                               static_cast<unsigned long long>(M) * caps.np1, C);
+    }
     const int d1 = ctx->tune_d1 >= 0 ? ctx->tune_d1 : 2;
     DevBuf cnt_buf, need;
     TRY(cnt_buf.alloc(ctx, sizeof(Counters)));
@@ -713,6 +942,14 @@ int direct_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const 
     int pmax = 0, amax = 0;
     TRY(known_max_row(ctx, P, &pmax));
     TRY(known_max_row(ctx, A, &amax));
+    ReplayCaps caps;
+    if (plain_tuning(ctx) && bounded_rows(true, R.max_row, amax, A.N, pmax, P.N, &caps)) {
+        RowRunner rr{ctx, true, kSymb, DirectRowArgs{view(R), view(A), view(P)}, {}, amax, pmax};
+        const long long s1 = std::min<long long>(static_cast<long long>(R.max_row) * amax, A.N);
+        const long long s2 = std::min<long long>(s1 * pmax, P.N);
+        return product_bounded(ctx, rr, M, P.N, flavour, out_vt, caps, s1, s2,
+                               static_cast<unsigned long long>(M) * s2, C);
+    }
     DevBuf cnt_buf, need, need_opt;
     TRY(cnt_buf.alloc(ctx, sizeof(Counters)));
     TRY(need.alloc(ctx, sizeof(int) * (static_cast<size_t>(M) + 1)));

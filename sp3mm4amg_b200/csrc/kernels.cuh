@@ -30,11 +30,22 @@ struct PairRowArgs {
     CsrView A, B;      // C = A*B, one output row per row of A
 };
 
+// Capacities of the replayed row kernels (rowreplay.cuh), per stage: products,
+// distinct columns and (stage 1) left steps of a row; np2 = ns2 = 0 for the
+// single-stage A*B.  Columns and steps are numbered in one byte.
+struct ReplayCaps {
+    int np1, ns1, k1, np2, ns2;
+};
+constexpr int kReplayMaxColumns = 256;
+// Booked output is handed to a warp this many entries at a time.
+constexpr int kReplayBook = 512;
+
 // Per-launch parameters shared by both row-kernel families.
 struct RowParams {
-    const int* rows;          // the rows of this launch
+    const int* rows;          // the rows of this launch (lanes kernels: nullptr = all)
     int nrows;
-    const int* nrows_dev;     // CTA-per-row kernel: row count on the device (set: nrows bounds it)
+    const int* nrows_dev;     // CTA-per-row and lanes kernels: row count on the device
+                              // (set: nrows bounds it)
     int S1, S2;               // table slots (powers of two >= 32); S2: direct only
     unsigned char* gtab;      // tables in global memory (nullptr: shared memory)
     long long gstride;        // bytes per group in gtab
@@ -60,6 +71,11 @@ struct RowParams {
     // left-row step (log2, at most 5, every right row at most that long), or
     // -1 for packed batches (any row length).
     int lg1, lg2;
+    // Replayed rows (every row 0 .. nrows-1, no list): capacities, and the
+    // rows left for another kernel.
+    ReplayCaps rcaps;
+    int* left_rows;
+    int* left_count;
 };
 
 // Launch geometry of one row-kernel launch.
@@ -82,6 +98,17 @@ cudaError_t launch_direct_rows(const DirectRowArgs& a, const RowParams& p, int m
 cudaError_t launch_direct_lanes(const DirectRowArgs& a, const RowParams& p, int mode,
                                 const RowGeom& geo, cudaStream_t st);
 size_t lanes_row_bytes(int mode, int S1, int S2);
+// The same for one SpMM row per warp (batch layout p.lg1).
+cudaError_t launch_pair_lanes(const PairRowArgs& a, const RowParams& p, int mode,
+                              const RowGeom& geo, cudaStream_t st);
+size_t pair_lanes_row_bytes(int mode, int S);
+// Rows of few products (rowreplay.cuh), one warp per row, consecutive rows
+// per warp.  replay_bytes: shared memory per warp.
+cudaError_t launch_direct_replay(const DirectRowArgs& a, const RowParams& p, int mode,
+                                 const RowGeom& geo, cudaStream_t st);
+cudaError_t launch_pair_replay(const PairRowArgs& a, const RowParams& p, int mode,
+                               const RowGeom& geo, cudaStream_t st);
+size_t replay_bytes(int mode, const ReplayCaps& c, int warps);
 // Tuning value of "lanes per row" that runs every direct row on the
 // CTA-per-row kernel.
 constexpr int kDenseLanes = 512;

@@ -762,7 +762,8 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
     p.retry_count = &dc->retry_count;
     p.err = ctx->d_err;
     p.c_vt = out_vt;
-    const bool replay = M >= kReplayMinRows && caps.np1 >= kReplayMinProducts;
+    const bool tiny = !rr.direct && caps.np1 <= kTinyProducts;
+    const bool replay = !tiny && M >= kReplayMinRows && caps.np1 >= kReplayMinProducts;
     DevBuf left;
     if (replay) TRY(left.alloc(ctx, sizeof(int) * (static_cast<size_t>(M) + 1)));
     int* n_left = left.as<int>() + M;
@@ -785,6 +786,17 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
     auto rows = [&](int mode) -> int {
         rr.mode = mode;
         RowParams q = p;
+        if (tiny) {
+            static const char* const kTiny[3] = {"pair.tiny.symb", "pair.tiny.num",
+                                                 "pair.tiny.book"};
+            q.S1 = caps.np1;
+            cudaError_t e = cudaSuccess;
+            prof(ctx, kTiny[mode], [&] { e = launch_pair_tiny(rr.pa, q, mode, st); });
+            if (e != cudaSuccess)
+                return set_error(ctx, SP3MM_ECUDA, "thread-per-row kernel launch failed: %s",
+                                 cudaGetErrorString(e));
+            return SP3MM_OK;
+        }
         if (replay) {
             CK(ctx, cudaMemsetAsync(n_left, 0, sizeof(int), st));
             const RowGeom geo = geometry(mode);
@@ -905,8 +917,8 @@ int spmm_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flav
                             (B.M ? static_cast<double>(B.nnz) / B.M : 0.0);
     if (ctx->tune_G == 0 && products <= 8.0) G = 4;
     ReplayCaps caps;
-    if (G == 32 && plain_tuning(ctx) &&
-        bounded_rows(false, A.max_row, B.max_row, B.N, 0, 0, &caps)) {
+    if (plain_tuning(ctx) && bounded_rows(false, A.max_row, B.max_row, B.N, 0, 0, &caps) &&
+        (G == 32 || caps.np1 <= kTinyProducts)) {
         RowRunner rr{ctx, false, kSymb, {}, PairRowArgs{view(A), view(B)}, -1, B.max_row};
         return product_bounded(ctx, rr, M, B.N, flavour, out_vt, caps,
                                std::min<long long>(caps.np1, B.N), 0,

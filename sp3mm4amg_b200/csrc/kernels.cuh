@@ -109,6 +109,11 @@ cudaError_t launch_direct_replay(const DirectRowArgs& a, const RowParams& p, int
 cudaError_t launch_pair_replay(const PairRowArgs& a, const RowParams& p, int mode,
                                const RowGeom& geo, cudaStream_t st);
 size_t replay_bytes(int mode, const ReplayCaps& c, int warps);
+// SpMM rows of at most p.S1 <= kTinyProducts products, one thread per row over
+// all rows (rowtiny.cuh).
+constexpr int kTinyProducts = 32;
+cudaError_t launch_pair_tiny(const PairRowArgs& a, const RowParams& p, int mode,
+                             cudaStream_t st);
 // Tuning value of "lanes per row" that runs every direct row on the
 // CTA-per-row kernel.
 constexpr int kDenseLanes = 512;

@@ -1,6 +1,6 @@
 """Products whose longest rows bound every row's products (no bounds pass, no
-binning): the replayed rows (rowreplay.cuh) and the lanes kernels over all
-rows or over what the replay leaves.
+binning): the replayed rows (rowreplay.cuh), the lanes kernels over all rows
+or over what the replay leaves, and the thread-per-row SpMM (rowtiny.cuh).
 Results must be bit-identical to the oracle and to the binned path (lane
 tuning takes it), in every flavour and value type."""
 import numpy as np
@@ -109,3 +109,18 @@ def test_one_column(orc):
     A = _rows(rng, 300, 1, 1, 1)
     R = _rows(rng, 16384, 300, 250, 256)
     _check(orc, [R, A], what="pair")
+
+
+@pytest.mark.parametrize("M", [1, 31, 33, 127, 128, 129, 1000])
+@pytest.mark.parametrize("k,l", [(8, 4), (31, 1), (1, 32), (3, 7)])
+def test_tiny_rows(orc, M, k, l):
+    rng = np.random.default_rng(100 * M + k)
+    _check(orc, [_rows(rng, M, 50, 0, k), _rows(rng, 50, 40, min(l, 1), l)], what=(M, k, l))
+
+
+def test_tiny_rows_all_distinct(orc):
+    # 32 products, 32 columns: the list at its capacity.
+    n = 32
+    A = S.CSR(np.array([0, 8, 16]), np.tile(np.arange(8), 2), np.arange(16.0) - 7, (2, 8))
+    B = S.CSR(np.arange(9) * 4, np.arange(n)[::1].astype(np.int64), np.arange(32.0) + 0.5, (8, n))
+    _check(orc, [A, B])

@@ -235,8 +235,15 @@ struct RowRunner {
         return avg >= 0.75 * (1 << lg) ? lg : -1;
     }
 
-    long long operand_nnz() const {
-        return direct ? da.R.nnz + da.A.nnz + da.P.nnz : pa.A.nnz + pa.B.nnz;
+    // Entries of booking space: SpMM results may hold several times their
+    // operands' nonzeros, Galerkin products (and the batches, which book by
+    // the same rule) a third of theirs.  Eight times those of a 128^3
+    // hierarchy's first product was 2.8 GB allocated and freed per build, and
+    // a program that holds its last hierarchy while it builds the next made
+    // the pool remap it: 30 ms a build against 24.
+    unsigned long long booked_entries() const {
+        return direct ? 2ULL * static_cast<unsigned long long>(da.R.nnz + da.A.nnz + da.P.nnz)
+                      : 8ULL * static_cast<unsigned long long>(pa.A.nnz + pa.B.nnz);
     }
 
     int launch(RowParams p, int G, DevBuf& gtab) {
@@ -683,8 +690,7 @@ int product_rows(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, int o
         const size_t eb = sizeof(int) + vbytes(out_vt);
         unsigned long long cap = std::min<unsigned long long>(
             bins.total,
-            std::max<unsigned long long>(1ULL << 20,
-                                         8ULL * static_cast<unsigned long long>(rr.operand_nnz())));
+            std::max<unsigned long long>(1ULL << 20, rr.booked_entries()));
         // Space the pool already holds idle is used without asking the
         // device for its free memory (a slow query).
         if (cap * eb > (size_t(1) << 30) && pool_idle_bytes(ctx) < cap * eb)
@@ -836,8 +842,7 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
         const size_t eb = sizeof(int) + vbytes(out_vt);
         unsigned long long cap = std::min<unsigned long long>(
             out_bound,
-            std::max<unsigned long long>(1ULL << 20,
-                                         8ULL * static_cast<unsigned long long>(rr.operand_nnz())));
+            std::max<unsigned long long>(1ULL << 20, rr.booked_entries()));
         if (cap * eb > (size_t(1) << 30) && pool_idle_bytes(ctx) < cap * eb)
             cap = std::min<unsigned long long>(
                 cap, std::max<unsigned long long>(1ULL << 20, free_device_bytes(ctx) / 2 / eb));

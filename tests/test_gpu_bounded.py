@@ -124,3 +124,17 @@ def test_tiny_rows_all_distinct(orc):
     A = S.CSR(np.array([0, 8, 16]), np.tile(np.arange(8), 2), np.arange(16.0) - 7, (2, 8))
     B = S.CSR(np.arange(9) * 4, np.arange(n)[::1].astype(np.int64), np.arange(32.0) + 0.5, (8, n))
     _check(orc, [A, B])
+
+
+@pytest.mark.parametrize("a_cols", [1, 600])
+def test_booking_space_overflows(orc, a_cols):
+    # More entries than the booking space holds (twice the operands', at
+    # least 2^20): the product is redone with symbolic sizes, on the bounded
+    # path (one product per row of R*A) and the binned one (600).
+    rng = np.random.default_rng(6)
+    R = _rows(rng, 2000, 1, 1, 1)
+    A = _rows(rng, 1, a_cols, a_cols, a_cols)
+    P = _rows(rng, a_cols, 600, 600 if a_cols == 1 else 1, 600 if a_cols == 1 else 1)
+    if a_cols > 1:
+        P = S.CSR(P.indptr, np.arange(600, dtype=np.int64), P.data, P.shape)
+    _check(orc, [R, A, P])

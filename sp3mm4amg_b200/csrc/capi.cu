@@ -1863,34 +1863,36 @@ int sp3mm_transpose(sp3mm_ctx* ctx, const sp3mm_dcsr* A, sp3mm_dcsr* AT) {
     if (!ctx || !AT) return SP3MM_EINVAL;
     TRY(check_dcsr(ctx, A, "A"));
     const cudaStream_t st = ctx->stream;
-    DevBuf rp, ci, v, counts, cursor;
-    TRY(counts.alloc(ctx, sizeof(int) * (static_cast<size_t>(A->N) + 1)));
-    TRY(cursor.alloc(ctx, sizeof(int) * (static_cast<size_t>(A->N) + 1)));
-    CK(ctx, cudaMemsetAsync(counts.p, 0, sizeof(int) * (static_cast<size_t>(A->N) + 1), st));
-    CK(ctx, cudaMemsetAsync(cursor.p, 0, sizeof(int) * (static_cast<size_t>(A->N) + 1), st));
-    launch_col_counts(A->nnz, A->col, counts.as<int>(), st);
-    long long nnz = 0;
-    TRY(scan_counts(ctx, A->N, counts.as<int>(), rp, &nnz));
+    // Column counts, their scan, a scatter in arbitrary order within a row
+    // and the rows' sort, which flags a column that A's row holds twice; one
+    // round trip at the end.
+    const int M = A->N;
+    const size_t words = static_cast<size_t>(M) + 1;
+    DevBuf rp, ci, v, work, tmp;
+    TRY(work.alloc(ctx, 2 * sizeof(int) * words));
+    int* counts = work.as<int>();
+    CK(ctx, cudaMemsetAsync(work.p, 0, 2 * sizeof(int) * words, st));
+    TRY(rp.alloc(ctx, rp_bytes(M)));
     TRY(ci.alloc(ctx, sizeof(int) * static_cast<size_t>(A->nnz)));
     TRY(v.alloc(ctx, vbytes(A->val_type) * static_cast<size_t>(A->nnz)));
-    launch_transpose_scatter(view(*A), rp.as<int>(), cursor.as<int>(), ci.as<int>(), v.p, st);
-    // The scatter order within a row is arbitrary: sort (the sort kernels
-    // skip the rows they do not handle, so they run without knowing the
-    // longest row), then validate, which also finds the longest row.
-    launch_sort_rows(A->N, rp.as<int>(), ci.as<int>(), v.p, A->val_type, INT_MAX, st);
+    const size_t tb = scan_temp_bytes(M);
+    TRY(tmp.alloc(ctx, tb));
+    launch_col_counts(A->nnz, A->col, counts, st);
+    launch_scan(M, counts, rp.as<int>(), tmp.p, tb, st);
+    int* mr = rp.as<int>() + M + 1;
+    CK(ctx, cudaMemsetAsync(mr, 0, sizeof(int), st));
+    launch_count_max(M, counts, nullptr, mr, st);
+    launch_transpose_scatter(view(*A), rp.as<int>(), counts + words, ci.as<int>(), v.p, st);
+    launch_sort_rows(M, rp.as<int>(), ci.as<int>(), v.p, A->val_type, INT_MAX, st, ctx->d_err);
     CK(ctx, cudaGetLastError());
-    DevBuf mr;
-    TRY(mr.alloc(ctx, sizeof(int)));
-    CK(ctx, cudaMemsetAsync(mr.p, 0, sizeof(int), st));
-    launch_validate_i32(A->N, A->M, rp.as<int>(), ci.as<int>(), mr.as<int>(), ctx->d_err, st);
-    int max_row = 0;
-    CK(ctx, cudaMemcpyAsync(&max_row, mr.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TRY(check_device_err(ctx));   // synchronises: max_row is complete
-    AT->M = A->N;
+    unsigned* box = ctx->host_box;
+    CK(ctx, cudaMemcpyAsync(box, mr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TRY(check_device_err(ctx));   // synchronises: box is complete
+    AT->M = M;
     AT->N = A->M;
     AT->nnz = A->nnz;
     AT->val_type = A->val_type;
-    AT->max_row = max_row;
+    AT->max_row = static_cast<int>(box[0]);
     return finish_matrix(AT, rp, ci, v);
 }
 

@@ -295,16 +295,19 @@ __global__ void k_col_counts(long long nnz, const int* ci, int* counts) {
         atomicAdd(counts + ci[i], 1);
 }
 
-__global__ void __launch_bounds__(256) k_transpose_scatter(CsrView A, const int* t_rp,
+// 2^lg lanes per row of A (its mean length: a warp per row of the four
+// entries of a fine prolongator took 0.41 ms at 128^3, four lanes 0.09).
+__global__ void __launch_bounds__(256) k_transpose_scatter(CsrView A, int lg, const int* t_rp,
                                                             int* cursor, int* t_ci, void* t_v) {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) / 32;
-    for (int row = (blockIdx.x * blockDim.x + threadIdx.x) / 32; row < A.M; row += warps) {
+    const int sub = threadIdx.x & ((1 << lg) - 1);
+    const long long groups = (static_cast<long long>(gridDim.x) * blockDim.x) >> lg;
+    for (long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> lg; row < A.M;
+         row += groups) {
         const int b = A.rp[row], e = A.rp[row + 1];
-        for (int j = b + lane; j < e; j += 32) {
+        for (int j = b + sub; j < e; j += 1 << lg) {
             const int c = A.ci[j];
             const int pos = t_rp[c] + atomicAdd(cursor + c, 1);
-            t_ci[pos] = row;
+            t_ci[pos] = static_cast<int>(row);
             if (A.vtype == SP3MM_F32)
                 static_cast<float*>(t_v)[pos] = static_cast<const float*>(A.v)[j];
             else
@@ -313,66 +316,77 @@ __global__ void __launch_bounds__(256) k_transpose_scatter(CsrView A, const int*
     }
 }
 
-// Rows of more than 32 and at most kSortSmemRow entries: a warp per row
-// sorts the row in shared memory with a bitonic network (the coarse levels'
-// restrictions hold rows of hundreds of entries; odd-even transposition in
-// global memory took 2.8 ms for the 512 rows of 677 entries of 128^3 level
-// 3).  Columns within a row are distinct, so the order is unique.
+// Rows of more than 32 and at most kSortSmemRow entries: a CTA per row counts
+// every column's rank (the row in shared memory, four columns compared per
+// load).  The coarse levels' restrictions hold rows of 84 to 677 entries: a
+// warp per row with a bitonic network took 1.13 ms over the levels of a 128^3
+// hierarchy, this 0.43.  A column met twice is flagged where err is given.
 constexpr int kSortSmemRow = 2048;
-constexpr int kSortSmemWarps = 4;
+constexpr int kSortThreads = 128;
 
-__global__ void __launch_bounds__(kSortSmemWarps * 32) k_sort_rows_smem(int M, const int* rp,
-                                                                        int* ci, void* v, int vt) {
-    extern __shared__ __align__(16) unsigned char sort_smem[];
+__global__ void __launch_bounds__(kSortThreads) k_sort_rows_cta(int M, int chunk, const int* rp,
+                                                                int* ci, void* v, int vt,
+                                                                unsigned* err) {
+    __shared__ __align__(16) int sk[kSortSmemRow + 4];
+    __shared__ double sv[kSortSmemRow];
+    constexpr int U = 4;   // columns a thread ranks together
     const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    double* sv = reinterpret_cast<double*>(sort_smem) + static_cast<size_t>(w) * kSortSmemRow;
-    int* sk = reinterpret_cast<int*>(reinterpret_cast<double*>(sort_smem) +
-                                     static_cast<size_t>(kSortSmemWarps) * kSortSmemRow) +
-              static_cast<size_t>(w) * kSortSmemRow;
-    const int warps = (gridDim.x * blockDim.x) / 32;
-    for (int row = (blockIdx.x * blockDim.x + threadIdx.x) / 32; row < M; row += warps) {
-        const int b = rp[row], e = rp[row + 1];
-        const int n = e - b;
-        if (n <= 32 || n > kSortSmemRow) continue;
-        int P2 = 64;
-        while (P2 < n) P2 <<= 1;
-        for (int i = lane; i < P2; i += 32) {
-            sk[i] = i < n ? ci[b + i] : INT_MAX;
-            sv[i] = i < n ? load_val(v, vt, b + i) : 0.0;
+    for (long long r0 = blockIdx.x * static_cast<long long>(chunk); r0 < M;
+         r0 += gridDim.x * static_cast<long long>(chunk)) {
+        // Every warp looks the chunk's (at most 32) lengths up.
+        int lb = 0, ln = 0;
+        if (lane < chunk && r0 + lane < M) {
+            lb = rp[r0 + lane];
+            ln = rp[r0 + lane + 1] - lb;
         }
-        __syncwarp();
-        for (int k = 2; k <= P2; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = lane; i < P2; i += 32) {
-                    const int ixj = i ^ j;
-                    if (ixj > i) {
-                        const int a0 = sk[i], a1 = sk[ixj];
-                        if ((a0 > a1) == ((i & k) == 0)) {
-                            sk[i] = a1;
-                            sk[ixj] = a0;
-                            const double x0 = sv[i];
-                            sv[i] = sv[ixj];
-                            sv[ixj] = x0;
+        unsigned rows = __ballot_sync(0xffffffffu, ln > 32 && ln <= kSortSmemRow);
+        for (; rows; rows &= rows - 1) {
+            const int b = __shfl_sync(0xffffffffu, lb, __ffs(rows) - 1);
+            const int n = __shfl_sync(0xffffffffu, ln, __ffs(rows) - 1);
+            for (int i = threadIdx.x; i < n; i += kSortThreads) {
+                sk[i] = ci[b + i];
+                sv[i] = load_val(v, vt, b + i);
+            }
+            if (threadIdx.x < 4) sk[n + threadIdx.x] = INT_MAX;
+            __syncthreads();
+            for (int i0 = threadIdx.x; i0 < n; i0 += U * kSortThreads) {
+                int k[U], lt[U], eq[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int i = i0 + u * kSortThreads;
+                    k[u] = i < n ? sk[i] : -1;
+                    lt[u] = eq[u] = 0;
+                }
+                for (int j = 0; j < n; j += 4) {
+                    const int4 q = *reinterpret_cast<const int4*>(sk + j);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (u * kSortThreads < n) {
+                            lt[u] += (q.x < k[u]) + (q.y < k[u]) + (q.z < k[u]) + (q.w < k[u]);
+                            eq[u] += (q.x == k[u]) + (q.y == k[u]) + (q.z == k[u]) + (q.w == k[u]);
                         }
                     }
                 }
-                __syncwarp();
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int i = i0 + u * kSortThreads;
+                    if (i < n) {
+                        ci[b + lt[u]] = k[u];
+                        store_val(v, vt, b + lt[u], sv[i]);
+                        if (eq[u] > 1 && err) atomicOr(err, kErrInput);
+                    }
+                }
             }
+            __syncthreads();
         }
-        for (int i = lane; i < n; i += 32) {
-            ci[b + i] = sk[i];
-            store_val(v, vt, b + i, sv[i]);
-        }
-        __syncwarp();
     }
 }
 
 // Sort each row's (col, val) by col.  Warp per row; rows up to 32 entries by
-// rank in registers, rows of k_sort_rows_smem's range there, longer rows by
+// rank in registers, rows of k_sort_rows_cta's range there, longer rows by
 // odd-even transposition in place.
 __global__ void __launch_bounds__(256) k_sort_rows(int M, const int* rp, int* ci, void* v,
-                                                    int vt) {
+                                                    int vt, unsigned* err) {
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) / 32;
     for (int row = (blockIdx.x * blockDim.x + threadIdx.x) / 32; row < M; row += warps) {
@@ -383,17 +397,22 @@ __global__ void __launch_bounds__(256) k_sort_rows(int M, const int* rp, int* ci
             const bool in = lane < n;
             const int k = in ? ci[b + lane] : INT_MAX;
             const double x = in ? load_val(v, vt, b + lane) : 0.0;
-            int r = 0;
-            for (int j = 0; j < n; ++j) r += __shfl_sync(0xffffffffu, k, j) < k;
+            int r = 0, eq = 0;
+            for (int j = 0; j < n; ++j) {
+                const int kj = __shfl_sync(0xffffffffu, k, j);
+                r += kj < k;
+                eq += kj == k;
+            }
             __syncwarp();
             if (in) {
                 ci[b + r] = k;
                 store_val(v, vt, b + r, x);
+                if (eq > 1 && err) atomicOr(err, kErrInput);
             }
             __syncwarp();
             continue;
         }
-        if (n <= kSortSmemRow) continue;   // k_sort_rows_smem
+        if (n <= kSortSmemRow) continue;   // k_sort_rows_cta
         for (int phase = 0; phase < n; ++phase) {
             for (int i = b + (phase & 1) + 2 * lane; i + 1 < e; i += 64) {
                 const int a0 = ci[i], a1 = ci[i + 1];
@@ -407,6 +426,9 @@ __global__ void __launch_bounds__(256) k_sort_rows(int M, const int* rp, int* ci
             }
             __syncwarp();
         }
+        if (err)
+            for (int i = b + lane; i + 1 < e; i += 32)
+                if (ci[i] == ci[i + 1]) atomicOr(err, kErrInput);
     }
 }
 
@@ -575,24 +597,25 @@ void launch_col_counts(long long nnz, const int* ci, int* counts, cudaStream_t s
 void launch_transpose_scatter(const CsrView& A, const int* t_rp, int* cursor, int* t_ci,
                               void* t_v, cudaStream_t st) {
     if (A.M == 0) return;
-    k_transpose_scatter<<<grid_for(static_cast<long long>(A.M) * 32, 256), 256, 0, st>>>(
-        A, t_rp, cursor, t_ci, t_v);
+    int lg = 0;
+    while (lg < 5 && (1LL << lg) * A.M < A.nnz) ++lg;   // mean row length
+    k_transpose_scatter<<<grid_for(static_cast<long long>(A.M) << lg, 256), 256, 0, st>>>(
+        A, lg, t_rp, cursor, t_ci, t_v);
     note_launch();
 }
 
 void launch_sort_rows(int M, const int* rp, int* ci, void* v, int vt, int max_row,
-                      cudaStream_t st) {
+                      cudaStream_t st, unsigned* err) {
     if (M == 0 || max_row <= 1) return;
-    k_sort_rows<<<grid_for(static_cast<long long>(M) * 32, 256), 256, 0, st>>>(M, rp, ci, v,
-                                                                              vt);
+    k_sort_rows<<<grid_for(static_cast<long long>(M) * 32, 256), 256, 0, st>>>(M, rp, ci, v, vt,
+                                                                              err);
     note_launch();
     if (max_row > 32) {
-        const int smem = kSortSmemWarps * kSortSmemRow * 12;
-        // A failure here surfaces as the launch's error (callers check it).
-        cudaFuncSetAttribute(k_sort_rows_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem);
-        k_sort_rows_smem<<<grid_for(static_cast<long long>(M) * 32, kSortSmemWarps * 32),
-                           kSortSmemWarps * 32, smem, st>>>(M, rp, ci, v, vt);
+        // Few rows: one per CTA; many: 32 lengths looked up at once.
+        const int ctas = 148 * 8;
+        const int chunk = M < ctas ? 1 : M / ctas < 32 ? M / ctas : 32;
+        k_sort_rows_cta<<<grid_for(M, chunk, ctas), kSortThreads, 0, st>>>(M, chunk, rp, ci, v,
+                                                                           vt, err);
         note_launch();
     }
 }

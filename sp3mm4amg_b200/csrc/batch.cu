@@ -73,6 +73,10 @@ __global__ void k_batch_bounds(const BItem* __restrict__ items, const long long*
         long long o = nd >> d1;
         const long long r = static_cast<long long>(ceil(8.0 * sqrt(static_cast<double>(u))));
         if (r < o) o = r;
+        // (rows of up to 64 products get tables for all of them: boundary rows
+        // of 7-point stencils hold more distinct columns than a quarter, and a
+        // retry round cost 0.1 ms of a 0.9 ms plan)
+        o = o > 64 ? o : (nd < 64 ? nd : 64);
         need_opt[g] = nd == 0 ? 0 : (u >= I->Y.N ? nd : max(1, static_cast<int>(o)));
         row_item[g] = lo;
         if (I->kind == kBatchDirect) {
@@ -133,6 +137,14 @@ __global__ void k_batch_local_rp(const BItem* __restrict__ items, const int* __r
     }
 }
 
+// Exact binning leaves out the rows that the replayed kernel does.
+__global__ void k_batch_drop_done(long long rows, const unsigned char* __restrict__ done,
+                                  int* need) {
+    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < rows;
+         g += (long long)gridDim.x * blockDim.x)
+        if (done[g]) need[g] = 0;
+}
+
 int grid_for_rows(long long rows) {
     long long g = (rows + 255) / 256;
     return static_cast<int>(std::max<long long>(1, std::min<long long>(g, 148LL * 32)));
@@ -175,6 +187,16 @@ struct sp3mm_batch {
     DevBuf d_items, d_bases, d_row_item, d_need, d_need_opt, d_cnt1, d_cnt2, d_crp;
     DevBuf d_ci, d_v, d_rp, d_rp_off, d_counters;
     DevBuf num_gtab;
+    // Replayed rows (rowreplay.cuh): runs of rows of the direct products with
+    // few products per row, in classes of one capacity, and which of their
+    // rows the plan's pass did.
+    struct Replay {
+        ReplayCaps caps;
+        int first, count;   // chunks
+    };
+    std::vector<int4> chunks;
+    std::vector<Replay> replays;
+    DevBuf d_chunks, d_done;
     Bins nbins;
     std::vector<BatchTier> tiers;
     std::vector<long long> rp_off;
@@ -185,8 +207,6 @@ struct sp3mm_batch {
     // Numeric graph (tiers as parallel branches).
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    std::vector<cudaStream_t> branch;
-    std::vector<cudaEvent_t> events;
     int graph_kernels = 0;
 
     ~sp3mm_batch() { drop_graph(); }
@@ -195,10 +215,6 @@ struct sp3mm_batch {
         if (graph) cudaGraphDestroy(graph);
         exec = nullptr;
         graph = nullptr;
-        for (auto s : branch) cudaStreamDestroy(s);
-        for (auto e : events) cudaEventDestroy(e);
-        branch.clear();
-        events.clear();
     }
 };
 
@@ -326,6 +342,9 @@ size_t gt_bytes(const BatchTier& t) {
     return static_cast<size_t>(t.grid) * (t.block / 32) * t.smem;
 }
 
+// The context's branch streams and events before these are the replayed rows'.
+constexpr int kTierStreams = 2, kTierEvents = 3;
+
 // Launch the tiers; with several, tier 0 runs on the context stream and the
 // others on branch streams forked from it and joined back (parallel graph
 // branches when captured).
@@ -334,21 +353,14 @@ int run_tiers(sp3mm_batch* b, int mode, const std::vector<BatchTier>& tiers, con
     sp3mm_ctx* ctx = b->ctx;
     const cudaStream_t st = ctx->stream;
     const int nt = static_cast<int>(tiers.size());
-    while (static_cast<int>(b->branch.size()) < nt - 1) {
-        cudaStream_t s;
-        CK(ctx, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        b->branch.push_back(s);
-    }
-    while (static_cast<int>(b->events.size()) < nt) {
-        cudaEvent_t e;
-        CK(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        b->events.push_back(e);
-    }
-    if (nt > 1) CK(ctx, cudaEventRecord(b->events[0], st));
+    TRY(need_branches(ctx, kTierStreams + std::max(nt - 1, 0), kTierEvents + nt));
+    const cudaStream_t* branch = ctx->branch.data() + kTierStreams - 1;   // of tier k > 0
+    const cudaEvent_t* event = ctx->branch_event.data() + kTierEvents;
+    if (nt > 1) CK(ctx, cudaEventRecord(event[0], st));
     for (int k = 0; k < nt; ++k) {
         const BatchTier& t = tiers[k];
-        const cudaStream_t s = k == 0 ? st : b->branch[k - 1];
-        if (k > 0) CK(ctx, cudaStreamWaitEvent(s, b->events[0], 0));
+        const cudaStream_t s = k == 0 ? st : branch[k];
+        if (k > 0) CK(ctx, cudaStreamWaitEvent(s, event[0], 0));
         BatchRowParams p = base;
         p.rows = lists + t.first;
         p.nrows = t.count;
@@ -368,10 +380,107 @@ int run_tiers(sp3mm_batch* b, int mode, const std::vector<BatchTier>& tiers, con
             CK(ctx, launch_batch_rows(mode, t.gt, b->tv, b->to, t.grid, t.block, smem, s,
                                       b->d_items.as<BItem>(), b->d_row_item.as<int>(), p));
         if (k > 0) {
-            CK(ctx, cudaEventRecord(b->events[k], s));
-            CK(ctx, cudaStreamWaitEvent(st, b->events[k], 0));
+            CK(ctx, cudaEventRecord(event[k], s));
+            CK(ctx, cudaStreamWaitEvent(st, event[k], 0));
         }
     }
+    return SP3MM_OK;
+}
+
+// The replayed kernel over the batch's chunks, on branches forked from the
+// context stream; join_replay() makes the context stream wait for them.
+int fork_replay(sp3mm_batch* b, int mode, const BatchRowParams& p) {
+    sp3mm_ctx* ctx = b->ctx;
+    if (b->replays.empty()) return SP3MM_OK;
+    TRY(need_branches(ctx, kTierStreams, kTierEvents));
+    CK(ctx, cudaEventRecord(ctx->branch_event[0], ctx->stream));
+    for (size_t k = 0; k < b->replays.size(); ++k) {
+        const auto& c = b->replays[k];
+        const cudaStream_t s = ctx->branch[k];
+        CK(ctx, cudaStreamWaitEvent(s, ctx->branch_event[0], 0));
+        const BatchReplay r{c.caps, b->to, b->d_done.as<unsigned char>(),
+                            b->d_need_opt.as<int>()};
+        CK(ctx, launch_batch_replay(mode, b->tv, c.count, s, b->d_items.as<BItem>(),
+                                    b->d_chunks.as<int4>() + c.first, p, r));
+        CK(ctx, cudaEventRecord(ctx->branch_event[k + 1], s));
+    }
+    return SP3MM_OK;
+}
+int join_replay(sp3mm_batch* b) {
+    for (size_t k = 0; k < b->replays.size(); ++k)
+        CK(b->ctx,
+           cudaStreamWaitEvent(b->ctx->stream, b->ctx->branch_event[k + 1], 0));
+    return SP3MM_OK;
+}
+
+// The direct products whose rows the replayed kernel may take, cut into runs
+// of rows for one wave of CTAs: X's longest row (where it is not known, its
+// mean) times Y's longest within kBoundedProducts, in two classes by the
+// kernel's unroll.  Rows past the capacities stay with the tiers.  20 grids of
+// 1e3 to 2e5 points: replayed numeric pass 0.73 -> 0.51 ms; booked plan 0.52 ->
+// 0.41 ms of kernels (one class for both sizes of rows: 0.47).
+int plan_replay(sp3mm_batch* b) {
+    sp3mm_ctx* ctx = b->ctx;
+    b->chunks.clear();
+    b->replays.clear();
+    auto steps = [](const BItem& I) {   // unknown: a quarter above the mean
+        if (I.xmax >= 0) return I.xmax;
+        return I.M > 0 ? static_cast<int>(std::min<long long>(1 << 20, I.X.nnz * 5 / 4 / I.M + 2))
+                       : 0;
+    };
+    auto products = [&](const BItem& I) -> long long {   // 0: not replayed
+        const long long p = static_cast<long long>(steps(I)) * I.ymax;
+        const bool ok = I.kind == kBatchDirect && I.M >= kReplayCtaRows && I.ymax >= 0 &&
+                        I.zmax >= 0 && steps(I) <= kReplayMaxColumns &&
+                        p >= kReplayMinProducts && p <= kBoundedProducts;
+        return ok ? p : 0;
+    };
+    long long all = 0;
+    for (const BItem& I : b->items) all += products(I) ? I.M : 0;
+    if (all < kReplayMinRows) return SP3MM_OK;
+    for (int k = 0; k < 2; ++k) {
+        long long rows = 0;
+        int np = 0, k1 = 0, n1 = 0, l2 = 0, n2 = 0, n = 0;
+        auto mine = [&](const BItem& I) {
+            const long long p = products(I);
+            return p > 0 && (p > kReplaySmall) == (k == 1);
+        };
+        for (const BItem& I : b->items) {
+            if (!mine(I)) continue;
+            ++n;
+            rows += I.M;
+            np = std::max(np, static_cast<int>(products(I)));
+            k1 = std::max(k1, steps(I));
+            n1 = std::max(n1, I.Y.N);
+            l2 = std::max(l2, I.zmax);
+            n2 = std::max(n2, I.N);
+        }
+        if (!n) continue;
+        sp3mm_batch::Replay c{replay_caps(true, np, k1, n1, l2, n2),
+                              static_cast<int>(b->chunks.size()), 0};
+        const size_t smem = replay_bytes(kNumBook, c.caps, kReplayWarps) + 1024;
+        const long long ctas =
+            std::max<long long>(1, std::min<long long>(replay_ctas(replay_unroll(c.caps)),
+                                                       ctx->smem_optin / smem)) *
+            ctx->num_sms;
+        // (each product may leave a shorter last run)
+        const long long full = std::max<long long>(1, ctas - n);
+        const long long per = std::max<long long>(kReplayCtaRows, (rows + full - 1) / full);
+        for (int i = 0; i < static_cast<int>(b->items.size()); ++i) {
+            if (!mine(b->items[i])) continue;
+            const long long M = b->items[i].M, parts = (M + per - 1) / per;
+            for (long long q = 0; q < parts; ++q)
+                b->chunks.push_back(make_int4(i, static_cast<int>(M * q / parts),
+                                              static_cast<int>(M * (q + 1) / parts), 0));
+        }
+        c.count = static_cast<int>(b->chunks.size()) - c.first;
+        b->replays.push_back(c);
+    }
+    TRY(b->d_done.alloc(ctx, static_cast<size_t>(b->rows)));
+    CK(ctx, cudaMemsetAsync(b->d_done.p, 0, static_cast<size_t>(b->rows), ctx->stream));
+    TRY(b->d_chunks.alloc(ctx, sizeof(int4) * b->chunks.size()));
+    CK(ctx, cudaMemcpyAsync(b->d_chunks.p, b->chunks.data(), sizeof(int4) * b->chunks.size(),
+                            cudaMemcpyHostToDevice, ctx->stream));
     return SP3MM_OK;
 }
 
@@ -399,19 +508,14 @@ int build_numeric(sp3mm_batch* b) {
     p.err = ctx->d_err;
     // Create branch streams and events before capture begins.
     const int nt = static_cast<int>(b->tiers.size());
-    while (static_cast<int>(b->branch.size()) < nt - 1) {
-        cudaStream_t s;
-        CK(ctx, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        b->branch.push_back(s);
-    }
-    while (static_cast<int>(b->events.size()) < nt) {
-        cudaEvent_t e;
-        CK(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        b->events.push_back(e);
-    }
+    TRY(need_branches(ctx, kTierStreams + std::max(nt - 1, 0), kTierEvents + nt));
+    // The replayed rows are parallel branches too.
     CK(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    const int rc = run_tiers(b, kNumExact, b->tiers, b->nbins.lists.as<int>(), p,
-                             b->num_gtab.as<unsigned char>());
+    int rc = fork_replay(b, kNumExact, p);
+    if (rc == SP3MM_OK)
+        rc = run_tiers(b, kNumExact, b->tiers, b->nbins.lists.as<int>(), p,
+                       b->num_gtab.as<unsigned char>());
+    if (rc == SP3MM_OK) rc = join_replay(b);
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(st, &g);
     if (rc != SP3MM_OK) {
@@ -421,7 +525,7 @@ int build_numeric(sp3mm_batch* b) {
     CK(ctx, e);
     b->graph = g;
     CK(ctx, cudaGraphInstantiate(&b->exec, g, 0));
-    b->graph_kernels = nt;
+    b->graph_kernels = nt + static_cast<int>(b->replays.size());
     return SP3MM_OK;
 }
 
@@ -505,6 +609,12 @@ int ensure_numeric(sp3mm_batch* b) {
     if (M > 0)
         launch_need_from_counts(M, b->d_cnt2.as<int>(), b->d_cnt1.as<int>(), b->d_need.as<int>(),
                                 ctx->stream);
+    if (M > 0 && !b->replays.empty()) {
+        k_batch_drop_done<<<grid_for_rows(M), 256, 0, ctx->stream>>>(
+            M, b->d_done.as<unsigned char>(), b->d_need.as<int>());
+        note_launch();
+        CK(ctx, cudaGetLastError());
+    }
     TRY(bin_rows(ctx, M, b->d_need.as<int>(), 0, 32, dc, nullptr, b->nbins));
     ProfSpan span(ctx, "batch.graph");
     return build_numeric(b);
@@ -555,9 +665,6 @@ int batch_plan(sp3mm_batch* b) {
         note_launch();
         CK(ctx, cudaGetLastError());
     }
-    Bins sb;
-    TRY(bin_rows(ctx, M, b->d_need_opt.as<int>(), 0, 32, dc, nullptr, sb));
-
     BatchRowParams p{};
     p.d1 = b->d1;
     p.d2 = b->d2;
@@ -566,12 +673,26 @@ int batch_plan(sp3mm_batch* b) {
     p.cnt1 = b->d_cnt1.as<int>();
     p.cnt2 = b->d_cnt2.as<int>();
     p.err = ctx->d_err;
+    TRY(plan_replay(b));
     bool booked = false;
+    Bins sb;
+    // The replayed rows first: the binning then leaves them out.
+    auto bin = [&](int mode, const BatchRowParams& q) -> int {
+        if (!b->replays.empty()) {
+            int rc = SP3MM_OK;
+            prof(ctx, "batch.replay", [&] {
+                rc = fork_replay(b, mode, q);
+                if (rc == SP3MM_OK) rc = join_replay(b);
+            });
+            TRY(rc);
+        }
+        return bin_rows(ctx, M, b->d_need_opt.as<int>(), 0, 32, dc, nullptr, sb);
+    };
     DevBuf ub_ci, ub_v, row_off, cursor;
     if (b->flavour == SP3MM_UB && rows > 0) {
         // One numeric pass: every row books its exact length from one
-        // cursor, in space bounded by the output bound, by twice the
-        // operands' nonzeros and by half the free memory (a batch that
+        // cursor, in space bounded by twice the operands' nonzeros (and a
+        // replaying warp's handout) and by half the free memory (a batch that
         // overflows it is planned symbolically instead).  Galerkin products
         // and their A*P0 steps write well under their operands' nonzeros;
         // reserving more made the pool map tens of GB for a batch of large
@@ -580,8 +701,8 @@ int batch_plan(sp3mm_batch* b) {
         long long in_nnz = 0;
         for (const BItem& I : b->items)
             in_nnz += I.X.nnz + I.Y.nnz + (I.kind == kBatchDirect ? I.Z.nnz : 0);
-        unsigned long long cap = std::min<unsigned long long>(
-            sb.total, std::max<unsigned long long>(1ULL << 20, 2ULL * in_nnz));
+        unsigned long long cap = std::max<unsigned long long>(1ULL << 20, 2ULL * in_nnz) +
+                                 b->chunks.size() * kReplayWarps * kReplayBook;
         if (cap * eb > (size_t(1) << 30) && pool_idle_bytes(ctx) < cap * eb)
             cap = std::min<unsigned long long>(
                 cap, std::max<unsigned long long>(1ULL << 20, free_device_bytes(ctx) / 2 / eb));
@@ -596,6 +717,7 @@ int batch_plan(sp3mm_batch* b) {
         q.row_off = row_off.as<long long>();
         q.ub_ci = ub_ci.as<int>();
         q.ub_v = ub_v.p;
+        TRY(bin(kNumBook, q));
         TRY(row_pass(b, kNumBook, sb, q, rinfo, "batch.book"));
         unsigned e = 0;
         TRY(read_err(ctx, &e));
@@ -609,7 +731,16 @@ int batch_plan(sp3mm_batch* b) {
             booked = true;
         }
     }
-    if (!booked && rows > 0) TRY(row_pass(b, kSymb, sb, p, rinfo, "batch.symbolic"));
+    if (!booked && rows > 0) {
+        // (after an overflow the rows are binned already, without those that
+        // the replayed kernel does)
+        if (b->flavour != SP3MM_UB) TRY(bin(kSymb, p));
+        else {
+            TRY(fork_replay(b, kSymb, p));
+            TRY(join_replay(b));
+        }
+        TRY(row_pass(b, kSymb, sb, p, rinfo, "batch.symbolic"));
+    }
 
     // Row pointers of the whole batch, product spans and longest rows.
     DevBuf tmp, span;
@@ -716,6 +847,8 @@ void batch_trim(sp3mm_batch* b) {
     b->d_cnt2.release();
     b->d_crp.release();
     b->d_rp_off.release();
+    b->d_chunks.release();
+    b->d_done.release();
     b->d_counters.release();
     b->num_gtab.release();
     b->nbins.level.release();
@@ -764,6 +897,8 @@ int sp3mm_batch_create(sp3mm_ctx* ctx, int n, const int* kinds, const sp3mm_dcsr
         I.kind = kinds[i] == SP3MM_BATCH_RAP ? kBatchDirect : kBatchPair;
         if (I.kind == kBatchDirect) I.Z = view(Z[i]);
         else I.Z = CsrView{};
+        I.xmax = X[i].max_row;
+        I.ymax = Y[i].max_row;
         I.zmax = I.kind == kBatchDirect ? Z[i].max_row : -1;
         I.M = X[i].M;
         I.N = I.kind == kBatchDirect ? Z[i].N : Y[i].N;

@@ -17,6 +17,7 @@ struct BItem {
     int kind;
     int M, N;              // shape of C
     long long row_base;    // first global row
+    int xmax, ymax;        // longest rows of X and Y (-1: unknown)
     int zmax;              // direct: longest row of Z (-1: unknown)
 };
 
@@ -49,6 +50,18 @@ struct BatchRowParams {
     int* ub_ci;
     void* ub_v;
 };
+
+// Replayed rows of a batch's direct products (rowreplay.cuh).
+struct BatchReplay {
+    ReplayCaps caps;
+    int to;                // output value type
+    unsigned char* done;   // per global row: replayed (set by the plan's pass)
+    int* need_zero;        // plan: table bound, zeroed for replayed rows
+};
+// CTA c takes rows [chunks[c].y, chunks[c].z) of product chunks[c].x.
+cudaError_t launch_batch_replay(int mode, int tv, int ctas, cudaStream_t st, const BItem* items,
+                                const int4* chunks, const BatchRowParams& p,
+                                const BatchReplay& r);
 
 // Sets the kernel's dynamic shared memory limit to `max_smem` and returns
 // how many CTAs of `block` threads with `smem` bytes each fit one SM.

@@ -114,6 +114,20 @@ size_t free_device_bytes(sp3mm_ctx* ctx) {
     return fr;
 }
 
+int need_branches(sp3mm_ctx* ctx, size_t streams, size_t events) {
+    while (ctx->branch.size() < streams) {
+        cudaStream_t s;
+        CK(ctx, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        ctx->branch.push_back(s);
+    }
+    while (ctx->branch_event.size() < events) {
+        cudaEvent_t e;
+        CK(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        ctx->branch_event.push_back(e);
+    }
+    return SP3MM_OK;
+}
+
 int read_err(sp3mm_ctx* ctx, unsigned* out) {
     CK(ctx, cudaMemcpyAsync(out, ctx->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost,
                             ctx->stream));
@@ -464,44 +478,14 @@ bool plain_tuning(const sp3mm_ctx* ctx) {
 // need no bounds pass and no binning: the bound sizes one launch over all
 // rows (a bounds launch, two binning launches and a host round trip fewer:
 // the 64x64 product 106 -> 85 us).
-constexpr int kBoundedProducts = 512;
-// Of these, products of at least kReplayMinRows rows with bounds of at least
-// kReplayMinProducts try the replayed rows (rowreplay.cuh) first.  Below that
-// many rows its templates serve too few (direct, 7-point box: 6,840 rows 87 us
-// against 57 on the lanes kernel alone, 21,000 rows 126 against 127, 262,144
-// rows 0.95 ms against 1.51); with fewer products a row is one batch of the
-// lanes kernel, and the rows of A*P alternate between patterns.
-constexpr int kReplayMinRows = 16384;
-constexpr int kReplayMinProducts = 48;
-// A CTA's rows share one template: as many as the resident CTAs leave, at
-// least this many (128 rows: 60 % slower at 50,000 rows of a 5-point grid).
-constexpr int kReplayCtaRows = 32;
-constexpr int kReplayWarps = 4;         // per CTA
-constexpr int kReplayCtasPerSm = 5;     // by registers
 
 // Whether rows of at most k1 steps of l1 products (and, direct, of P rows of
-// at most l2) are bounded so, and the replayed kernel's capacities: columns
-// and stage-2 products are optimistic (7-point R*A rows: 224 products, 79
-// columns, 316 stage-2 products; a template that does not fit leaves its rows
-// to the lanes kernel).
+// at most l2) are bounded so, and the replayed kernel's capacities.
 bool bounded_rows(bool direct, int k1, int l1, int n1, int l2, int n2, ReplayCaps* c) {
     if (k1 < 0 || l1 < 0 || l2 < 0 || k1 > kReplayMaxColumns) return false;
     const long long np = static_cast<long long>(k1) * l1;
     if (np > kBoundedProducts) return false;
-    auto columns = [](int p, int n) {
-        const int c = p <= 96 ? p : std::max(96, p / 2);
-        return std::max(1, std::min({c, n, kReplayMaxColumns}));
-    };
-    c->np1 = std::max(4, static_cast<int>(np + 3) / 4 * 4);
-    c->k1 = std::max(1, k1);
-    c->ns1 = columns(c->np1, n1);
-    c->np2 = c->ns2 = 0;
-    if (direct) {
-        const long long np2 =
-            std::min<long long>(static_cast<long long>(c->ns1) * l2, c->np1 * 3 / 2);
-        c->np2 = std::max(4, static_cast<int>(np2 + 3) / 4 * 4);
-        c->ns2 = std::max(1, std::min(c->ns1 <= 64 ? c->ns1 : std::max(64, c->ns1 / 2), n2));
-    }
+    *c = replay_caps(direct, static_cast<int>(np), k1, n1, l2, n2);
     return true;
 }
 
@@ -778,7 +762,8 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
         geo.block = 32 * kReplayWarps;
         geo.smem = replay_bytes(mode, caps, kReplayWarps);
         const long long per_sm = std::max<long long>(
-            1, std::min<long long>(kReplayCtasPerSm, ctx->smem_optin / (geo.smem + 1024)));
+            1, std::min<long long>(replay_ctas(replay_unroll(caps)),
+                                   ctx->smem_optin / (geo.smem + 1024)));
         geo.grid = static_cast<int>(std::min<long long>(
             (M + kReplayCtaRows - 1) / kReplayCtaRows, per_sm * ctx->num_sms));
         return geo;
@@ -1629,6 +1614,8 @@ int sp3mm_ctx_destroy(sp3mm_ctx* ctx) {
     if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+    for (auto s : ctx->branch) cudaStreamDestroy(s);
+    for (auto e : ctx->branch_event) cudaEventDestroy(e);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     pinned_cache().give(ctx->host_stage, ctx->host_stage_bytes);
     if (ctx->host_box) cudaFreeHost(ctx->host_box);

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -37,6 +38,12 @@ struct sp3mm_ctx {
     size_t free_at_check = 0;
     uint64_t reserved_at_check = 0;
     double free_checked_s = -1.0;
+    // Branch streams and events of the batches' parallel launches (creating
+    // them per batch took longer than its small launches): the first two
+    // streams and three events for the replayed rows, the others for the
+    // tiers.  Grown on demand, kept until the context is destroyed.
+    std::vector<cudaStream_t> branch;
+    std::vector<cudaEvent_t> branch_event;
     // Pinned host staging for downloads (grown on demand, freed with the
     // context).
     void* host_stage = nullptr;
@@ -167,6 +174,30 @@ struct Bins {
     DevBuf level, lists;
 };
 
+// Most products of a row on the replayed kernel, and of a row whose launch is
+// sized without a bounds pass.
+constexpr int kBoundedProducts = 512;
+
+// The replayed kernel's capacities for rows of `np` products in k1 steps,
+// columns below n1 (and, direct, P rows of at most l2 entries, columns below
+// n2).  Columns and stage-2 products are optimistic (7-point R*A rows: 224
+// products, 79 columns, 316 stage-2 products); a template that does not fit
+// leaves its rows to the table kernels.
+inline ReplayCaps replay_caps(bool direct, int np, int k1, int n1, int l2, int n2) {
+    ReplayCaps c{};
+    c.np1 = std::max(4, (np + 3) / 4 * 4);
+    c.k1 = std::max(1, k1);
+    c.ns1 = std::max(1, std::min({c.np1 <= 96 ? c.np1 : std::max(96, c.np1 / 2), n1,
+                                  kReplayMaxColumns}));
+    if (direct) {
+        const long long np2 =
+            std::min<long long>(static_cast<long long>(c.ns1) * l2, c.np1 * 3 / 2);
+        c.np2 = std::max(4, static_cast<int>(np2 + 3) / 4 * 4);
+        c.ns2 = std::max(1, std::min(c.ns1 <= 64 ? c.ns1 : std::max(64, c.ns1 / 2), n2));
+    }
+    return c;
+}
+
 // Device memory available to new allocations: free HBM plus the idle part
 // of the device's memory pool.
 size_t free_device_bytes(sp3mm_ctx* ctx);
@@ -178,6 +209,8 @@ size_t pool_idle_bytes(sp3mm_ctx* ctx);
 // takes 0.1-0.3 s per growth step and holds up the process's other threads'
 // CUDA calls meanwhile.  Failure is not an error (the pool grows on demand).
 void pool_reserve(sp3mm_ctx* ctx, size_t bytes);
+// At least `streams` branch streams and `events` events on the context.
+int need_branches(sp3mm_ctx* ctx, size_t streams, size_t events);
 int read_err(sp3mm_ctx* ctx, unsigned* out);
 // Read and clear the sticky device error word; map it to a return code.
 int check_device_err(sp3mm_ctx* ctx);

@@ -39,6 +39,23 @@ struct ReplayCaps {
 constexpr int kReplayMaxColumns = 256;
 // Booked output is handed to a warp this many entries at a time.
 constexpr int kReplayBook = 512;
+// Launches of at least kReplayMinRows rows with bounds of at least
+// kReplayMinProducts try the replayed rows.  Below that many rows the
+// templates serve too few (direct, 7-point box: 6,840 rows 87 us against 57
+// on the lanes kernel alone, 21,000 rows 126 against 127, 262,144 rows 0.95 ms
+// against 1.51); with fewer products a row is one batch of the lanes kernel,
+// and the rows of A*P alternate between patterns.
+constexpr int kReplayMinRows = 16384;
+constexpr int kReplayMinProducts = 48;
+// A CTA's rows share one template: as many as the resident CTAs leave, at
+// least this many (128 rows: 60 % slower at 50,000 rows of a 5-point grid).
+constexpr int kReplayCtaRows = 32;
+constexpr int kReplayWarps = 4;         // per CTA
+// Batches of products loaded together, and the CTAs per SM that the registers
+// leave: rows of up to kReplaySmall products have no use for four.
+constexpr int kReplaySmall = 128;
+constexpr int replay_unroll(const ReplayCaps& c) { return c.np1 <= kReplaySmall ? 2 : 4; }
+constexpr int replay_ctas(int unroll) { return unroll == 2 ? 8 : 5; }
 
 // Per-launch parameters shared by both row-kernel families.
 struct RowParams {
@@ -76,6 +93,8 @@ struct RowParams {
     ReplayCaps rcaps;
     int* left_rows;
     int* left_count;
+    unsigned char* done;      // a batch: rows replayed (in place of the list),
+    int* need_zero;           // and their table bounds, zeroed
 };
 
 // Launch geometry of one row-kernel launch.

@@ -36,6 +36,7 @@
 // per warp (1.1: half the warps).
 #pragma once
 
+#include "batch.cuh"
 #include "rowwarp.cuh"
 
 namespace sp3mm {
@@ -312,10 +313,10 @@ __device__ __forceinline__ bool replay_template(const Left& L, int n, const int*
 // a row outside the mask, the other row's, so that what is loaded through it
 // is in bounds; its results are not used), val(t) stores both rows' values of
 // that step to lv where they are not there yet.  Returns the rows that the
-// template describes up to shift[i]; sx.prod holds their products.  Lanes
-// past the end repeat the last step or product: loads and stores need no
-// branches.
-template <bool NUM, typename TB, class Key, class Val>
+// template describes up to shift[i]; sx.prod holds their products.  U batches of
+// products are loaded together.  Lanes past the end repeat the last step or
+// product: loads and stores need no branches.
+template <int U, bool NUM, typename TB, class Key, class Val>
 __device__ __forceinline__ unsigned replay_block(unsigned mask, const ReplayStage& st, Key&& key,
                                                  Val&& val, const double2* lv,
                                                  const int* __restrict__ rp,
@@ -339,7 +340,6 @@ __device__ __forceinline__ unsigned replay_block(unsigned mask, const ReplayStag
     if (!mask) return 0;
     shift[0] = shift[1] = 0;
     bad = 0;
-    constexpr int U = 4;   // batches loaded together
     for (int p0 = 0; p0 < st.np; p0 += 32 * U) {
         int p[U], k[U], c0[U], c1[U];
         TB v0[U], v1[U];
@@ -469,11 +469,23 @@ __device__ __forceinline__ void replay_write(unsigned mask, const ReplayStage& s
     }
 }
 
+// Mark the pair's rows of `did` as done (a batch: their table bound becomes
+// 0, so that no table kernel takes them).
+__device__ __forceinline__ void replay_mark(const RowParams& p, int row, unsigned did) {
+    const int lane = threadIdx.x & 31;
+    if (lane < 2 && (did >> lane & 1)) {
+        p.done[row + lane] = 1;
+        p.need_zero[row + lane] = 0;
+    }
+}
+
 // The rows [c0, c1) of this CTA in pairs dealt out to its warps, block(row,
 // mask, starts) for each with the rows' starts (and end) in rp loaded one
-// pair ahead; rows that it did not do are listed.  A warp most of whose first
-// pairs the template did not describe lists the rest untried.
-template <class Block>
+// pair ahead.  Rows that it did not do are listed, or (a batch's plan) those
+// it did are marked; a warp most of whose first pairs the template did not
+// describe leaves the rest untried.  DONE: only rows marked before, all of
+// which it has to do (a batch's replayed numeric pass).
+template <bool DONE, class Block>
 __device__ __forceinline__ void replay_rows(const RowParams& p, const int* __restrict__ rp,
                                             int c0, int c1, Block&& block) {
     constexpr int kTries = 8;   // rows before a warp may give up
@@ -484,7 +496,8 @@ __device__ __forceinline__ void replay_rows(const RowParams& p, const int* __res
 #pragma unroll
     for (int i = 0; i < 3; ++i) next[i] = __ldg(rp + min(row + i, p.nrows));
     for (; row < c1; row += step) {
-        if (tried >= kTries && 2 * hits < tried) {
+        if (!DONE && tried >= kTries && 2 * hits < tried) {
+            if (p.done) return;
             // This warp's remaining rows: whole pairs, and perhaps a last one.
             const int pairs = (c1 - row + step - 1) / step;
             const int n = 2 * pairs - (row + (pairs - 1) * step + 1 < c1 ? 0 : 1);
@@ -501,11 +514,20 @@ __device__ __forceinline__ void replay_rows(const RowParams& p, const int* __res
             at[i] = next[i];
             next[i] = __ldg(rp + min(row + step + i, p.nrows));
         }
-        const unsigned todo = row + 1 < c1 ? 3u : 1u;
-        const unsigned left = todo & ~block(row, todo, at);
+        unsigned todo = row + 1 < c1 ? 3u : 1u;
+        if (DONE) {
+            todo = __ballot_sync(kFull, lane < 2 && (todo >> lane & 1) && p.done[row + lane]);
+            if (!todo) continue;
+        }
+        const unsigned did = todo & block(row, todo, at);
+        const unsigned left = todo & ~did;
         tried += __popc(todo);
-        hits += __popc(todo & ~left);
-        if (left) {
+        hits += __popc(did);
+        if (DONE) {
+            if (left && lane == 0) atomicOr(p.err, kErrCount);   // the pattern has changed
+        } else if (p.done) {
+            replay_mark(p, row, did);
+        } else if (left) {
             int to = 0;
             if (lane == 0) to = atomicAdd(p.left_count, __popc(left));
             to = __shfl_sync(kFull, to, 0);
@@ -550,8 +572,10 @@ __device__ __forceinline__ void replay_share(ReplayStage& st, int (&box)[3]) {
     st.nst = box[2];
 }
 
-template <int MODE, typename TV, typename TO>
-__global__ void __launch_bounds__(128, 5) k_direct_replay(DirectRowArgs a, RowParams p) {
+// The rows [c0, c1) of a direct product by one CTA.
+template <int U, int MODE, bool DONE, typename TV, typename TO>
+__device__ __forceinline__ void replay_direct(const DirectRowArgs& a, const RowParams& p, int c0,
+                                              int c1) {
     constexpr bool NUM = MODE != kSymb;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int box[2][3];
@@ -561,9 +585,6 @@ __global__ void __launch_bounds__(128, 5) k_direct_replay(DirectRowArgs a, RowPa
     const TV* rv = static_cast<const TV*>(a.R.v);
     const TV* av = static_cast<const TV*>(a.A.v);
     const TV* pv = static_cast<const TV*>(a.P.v);
-    const int c0 = static_cast<int>(static_cast<long long>(p.nrows) * blockIdx.x / gridDim.x);
-    const int c1 =
-        static_cast<int>(static_cast<long long>(p.nrows) * (blockIdx.x + 1) / gridDim.x);
     replay_place(p.rcaps, NUM, blockDim.x >> 5, threadIdx.x >> 5, smem, st, &sx);
     if (threadIdx.x < 32 && c0 < c1) {
         const int row = replay_pick(a.R.rp, c0, c1);
@@ -576,12 +597,12 @@ __global__ void __launch_bounds__(128, 5) k_direct_replay(DirectRowArgs a, RowPa
     replay_share(st[0], box[0]);
     replay_share(st[1], box[1]);
     ReplayBook book;
-    replay_rows(p, a.R.rp, c0, c1, [&](int row, unsigned mask, const int (&at)[3]) -> unsigned {
+    replay_rows<DONE>(p, a.R.rp, c0, c1, [&](int row, unsigned mask, const int (&at)[3]) -> unsigned {
         if (st[0].nst < 0) return 0;
         int rb[2], sh1[2], sh2[2];
         mask = replay_starts(at, mask, st[0].nst, rb);
         if (!mask) return 0;
-        mask = replay_block<NUM>(
+        mask = replay_block<U, NUM>(
             mask, st[0], [&](int i, int t) { return __ldg(a.R.ci + rb[i] + t); },
             [&](int t) { sx.ss[t] = make_double2(ldv(rv, rb[0] + t), ldv(rv, rb[1] + t)); },
             sx.ss, a.A.rp, a.A.ci, av, sx, sh1);
@@ -595,7 +616,7 @@ __global__ void __launch_bounds__(128, 5) k_direct_replay(DirectRowArgs a, RowPa
         }
         if (!(mask & 1)) sh1[0] = sh1[1];
         if (!(mask & 2)) sh1[1] = sh1[0];
-        mask = replay_block<NUM>(
+        mask = replay_block<U, NUM>(
             mask, st[1], [&](int i, int t) { return st[0].sc[t] + sh1[i]; }, [](int) {}, sx.rav,
             a.P.rp, a.P.ci, pv, sx, sh2);
         if (mask) {
@@ -607,8 +628,51 @@ __global__ void __launch_bounds__(128, 5) k_direct_replay(DirectRowArgs a, RowPa
     });
 }
 
-template <int MODE, typename TV, typename TO>
-__global__ void __launch_bounds__(128, 5) k_pair_replay(PairRowArgs a, RowParams p) {
+template <int U, int MODE, typename TV, typename TO>
+__global__ void __launch_bounds__(128, replay_ctas(U)) k_direct_replay(DirectRowArgs a, RowParams p) {
+    const int c0 = static_cast<int>(static_cast<long long>(p.nrows) * blockIdx.x / gridDim.x);
+    const int c1 =
+        static_cast<int>(static_cast<long long>(p.nrows) * (blockIdx.x + 1) / gridDim.x);
+    replay_direct<U, MODE, false, TV, TO>(a, p, c0, c1);
+}
+
+// Runs of rows of a batch's direct products: CTA c takes rows [y, z) of
+// product chunks[c].x.
+template <int U, int MODE, typename TV, typename TO>
+__global__ void __launch_bounds__(128, replay_ctas(U))
+    k_batch_replay(const BItem* __restrict__ items, const int4* __restrict__ chunks,
+                   BatchRowParams b, BatchReplay r) {
+    const int4 ch = chunks[blockIdx.x];
+    const BItem* I = items + ch.x;
+    const long long g = I->row_base;
+    const DirectRowArgs a{I->X, I->Y, I->Z};
+    RowParams p{};
+    p.nrows = I->M;
+    p.c_vt = r.to;
+    p.err = b.err;
+    p.rcaps = r.caps;
+    p.done = r.done + g;
+    if (MODE == kNumExact) {
+        p.c_rp = b.c_rp + g;
+        p.c_ci = b.c_ci;
+        p.c_v = b.c_v;
+    } else {
+        p.need_zero = r.need_zero + g;
+        p.row_cnt = b.cnt2 + g;
+        p.row_cnt1 = b.cnt1 + g;
+        if (MODE == kNumBook) {
+            p.cursor = b.cursor;
+            p.cap = b.cap;
+            p.row_off = b.row_off + g;
+            p.ub_ci = b.ub_ci;
+            p.ub_v = b.ub_v;
+        }
+    }
+    replay_direct<U, MODE, MODE == kNumExact, TV, TO>(a, p, ch.y, ch.z);
+}
+
+template <int U, int MODE, typename TV, typename TO>
+__global__ void __launch_bounds__(128, replay_ctas(U)) k_pair_replay(PairRowArgs a, RowParams p) {
     constexpr bool NUM = MODE != kSymb;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int box[3];
@@ -629,12 +693,12 @@ __global__ void __launch_bounds__(128, 5) k_pair_replay(PairRowArgs a, RowParams
     }
     replay_share(st[0], box);
     ReplayBook book;
-    replay_rows(p, a.A.rp, c0, c1, [&](int row, unsigned mask, const int (&at)[3]) -> unsigned {
+    replay_rows<false>(p, a.A.rp, c0, c1, [&](int row, unsigned mask, const int (&at)[3]) -> unsigned {
         if (st[0].nst < 0) return 0;
         int ab[2], sh[2];
         mask = replay_starts(at, mask, st[0].nst, ab);
         if (!mask) return 0;
-        mask = replay_block<NUM>(
+        mask = replay_block<U, NUM>(
             mask, st[0], [&](int i, int t) { return __ldg(a.A.ci + ab[i] + t); },
             [&](int t) { sx.ss[t] = make_double2(ldv(avals, ab[0] + t), ldv(avals, ab[1] + t)); },
             sx.ss, a.B.rp, a.B.ci, bvals, sx, sh);

@@ -138,3 +138,41 @@ def test_booking_space_overflows(orc, a_cols):
     if a_cols > 1:
         P = S.CSR(P.indptr, np.arange(600, dtype=np.int64), P.data, P.shape)
     _check(orc, [R, A, P])
+
+
+@pytest.mark.parametrize("vt", [S.F64, S.F32])
+@pytest.mark.parametrize("fl", [S.UB, S.SYMBNUM])
+def test_batches(fl, vt):
+    # Batches whose direct products are replayed (2D and 3D stencils, broken
+    # patterns, fewer rows than a run) beside others (SpMM, heavy rows): equal
+    # to the single products, also after new values.
+    rng = np.random.default_rng(8)
+    probs = [pb.stencil_problem(len(d), d) for d in
+             [(170, 165), (41, 38, 35), (300, 120), (11, 9), (9, 8, 7), (64, 61), (47, 45, 40)]]
+    ops = [[p.R, p.A, p.P] for p in probs]
+    m = ops[2][1].to_scipy().copy()
+    m.data[rng.random(m.nnz) < 0.01] = 0.0
+    m.eliminate_zeros()
+    ops[2][1] = S.CSR.from_scipy(m)
+    ops.append([_rows(rng, 300, 400, 0, 40), _rows(rng, 400, 500, 0, 60), _rows(rng, 500, 90, 1, 9)])
+    with S.Context() as ctx:
+        for direct_only in (True, False):
+            d = [[ctx.upload(_random_values(x, rng), vt) for x in o] for o in ops]
+            if not direct_only:
+                d.append([ctx.upload(_random_values(x, rng), vt) for x in ops[0][:2]])
+            b = ctx.batch([tuple(x) for x in d], vt, fl)
+            b.run()
+            for step in range(2):
+                for i, x in enumerate(d):
+                    C = (ctx.rap(*x, S.DIRECT, S.UB, vt) if len(x) == 3 else
+                         ctx.spmm(*x, S.UB, vt))
+                    _equal(b.result(i).download(), C.download(), (direct_only, step, i))
+                    C.free()
+                for x in d:
+                    x[1].set_values(rng.uniform(-1, 1, x[1].nnz).astype(
+                        np.float64 if vt == S.F64 else np.float32).astype(np.float64))
+                b.run()          # replays the numeric pass with the new values
+            b.free()
+            for x in d:
+                for y in x:
+                    y.free()

@@ -41,9 +41,9 @@ __global__ void __launch_bounds__(kDWarps * 32, 1)
     k_batch_dense(const BItem* __restrict__ items, const int* __restrict__ row_item,
                   BatchRowParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int s_n1, s_lo, s_hi, s_cnt[kDWarps];
+    __shared__ int s_n1, s_lo, s_hi, s_cnt[kDWarps], s_pages;
     __shared__ long long s_base;
-    const DenseSmem d = dense_smem(smem, &s_n1, &s_lo, &s_hi, s_cnt, &s_base);
+    const DenseSmem d = dense_smem(smem, &s_n1, &s_lo, &s_hi, s_cnt, &s_pages, &s_base);
     dense_clear(d);
     const int nrows = p.nrows_dev ? *p.nrows_dev : p.nrows;
     for (long long it = blockIdx.x; it < nrows; it += gridDim.x) {

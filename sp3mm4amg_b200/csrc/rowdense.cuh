@@ -13,8 +13,14 @@
 //
 // Stage 1 (the R*A row) steps through the left entries: the CTA takes one
 // right row per step (a right row's columns are distinct, so a step has no
-// conflicts) and synchronises between steps (dstage1).  It walks the row's
-// column span in chunks of kDSpan columns.  Each column's first touch is
+// conflicts) and synchronises between steps (dstage1).  A row whose column
+// span exceeds the slice (its columns are runs in several grid planes) has
+// the slice paged: runs of 8 or more columns get a page of it as they are
+// first met, found through a page table over the span (128^3 level 2, rows
+// of 1,600 of 13,500 columns: 8.8 -> 6.1 ms for 4,096 rows, whose steps were
+// walked four times).  Only a row that
+// meets more pages than the slice holds walks its span in chunks of kDSpan
+// columns, over all products for each.  Each column's first touch is
 // recorded as the flat position of the product that made it (left
 // position, then right-row entry), and after each chunk the touched columns
 // are listed with their position and value.  Sorting that list by position
@@ -66,8 +72,13 @@ constexpr int kDSamples = 2048;   // columns sampled per stage for that histogra
 constexpr int kDSearch = 4;    // arity of the segment searches
 constexpr int kDSteps = kDWarps * 32;   // stage-1 left entries described at a time
 constexpr int kDAhead = 4;     // stage-1 steps whose products a thread loads ahead
-// The stage-1 step descriptions live over the warps' stage-2 staging.
-static_assert(kDSteps * 20 <= kDWarps * kDStage * 16, "step descriptions exceed the staging");
+constexpr int kDPages = 4096;  // page-table entries of a paged stage 1
+// The page table lies over the lists, which are written after the stage's steps.
+static_assert(kDPages * 4 <= kDList * 16, "page table exceeds the lists");
+// The stage-1 step descriptions and the pages' columns live over the warps'
+// stage-2 staging.
+static_assert(kDSteps * 20 + kDSpan / 8 * 4 <= kDWarps * kDStage * 16,
+              "step descriptions exceed the staging");
 
 // Dynamic shared memory: acc double[kDSpan] | ftq int[kDSpan] (after stage 1:
 // u64 sort keys [kDList]) | lkey int[kDList] | lq int[kDList] |
@@ -304,6 +315,9 @@ struct DenseSmem {
     int* sst;
     int* step;   // stage-1 step descriptions (over the warps' staging)
     int* hist;
+    int* pt;     // page table (over the lists)
+    int* pcol;   // first column of each page (over the staging, after the steps)
+    int* s_pages;
     long long* s_tot;
     int* s_n1;
     int* s_lo;
@@ -313,7 +327,8 @@ struct DenseSmem {
 };
 
 __device__ __forceinline__ DenseSmem dense_smem(unsigned char* smem, int* s_n1, int* s_lo,
-                                                int* s_hi, int* s_cnt, long long* s_base) {
+                                                int* s_hi, int* s_cnt, int* s_pages,
+                                                long long* s_base) {
     DenseSmem d;
     d.acc = reinterpret_cast<double*>(smem);
     d.ftq = reinterpret_cast<int*>(d.acc + kDSpan);
@@ -329,6 +344,9 @@ __device__ __forceinline__ DenseSmem dense_smem(unsigned char* smem, int* s_n1, 
     d.step = reinterpret_cast<int*>(d.touched + kDSpan);
     d.hist = reinterpret_cast<int*>(d.touched + kDSpan + static_cast<size_t>(kDWarps) * kDStage * 16);
     d.s_tot = reinterpret_cast<long long*>(d.hist + kDHist);
+    d.pt = d.lkey;
+    d.pcol = d.step + kDSteps * 5;
+    d.s_pages = s_pages;
     d.s_n1 = s_n1;
     d.s_lo = s_lo;
     d.s_hi = s_hi;
@@ -407,6 +425,31 @@ __device__ __forceinline__ void balanced_range(const DenseSmem& d, const Left& L
     __syncthreads();
 }
 
+// The slot of column c in a paged slice: its page's entry in the table pt over
+// the span from cb, a new page on first meeting (one per page among a warp's
+// lanes; a page that two warps claim at once is left unused by the second).
+// -1 when the pages ran out.
+__device__ __forceinline__ int dpage_slot(const DenseSmem& d, int c, int cb, int sh) {
+    const int i = (c - cb) >> sh;
+    int pg = d.pt[i];
+    if (pg < 0) {
+        const unsigned act = __activemask();
+        const unsigned same = __match_any_sync(act, i);
+        const int lead = __ffs(same) - 1;
+        if ((threadIdx.x & 31) == lead) {
+            const int id = atomicAdd(d.s_pages, 1);
+            if (id < kDSpan >> sh) {
+                d.pcol[id] = cb + (i << sh);
+                pg = atomicCAS(d.pt + i, -1, id);
+                if (pg < 0) pg = id;
+            }
+        }
+        pg = __shfl_sync(same, pg, lead);
+        if (pg < 0) return -1;
+    }
+    return (pg << sh) + ((c - cb) & ((1 << sh) - 1));
+}
+
 // Stage 1 (the R*A row) over the columns [cb, ce) of the slice starting at
 // cb, one left entry (step) at a time: the whole CTA takes step t's right
 // row (thread i its entries i, i + blockDim, ...), adds the rounded products
@@ -424,9 +467,12 @@ __device__ __forceinline__ void balanced_range(const DenseSmem& d, const Left& L
 // row, at most all):
 // they synchronise among themselves with a named barrier, so warps that
 // would idle add nothing to a step's cost.
-template <bool NUM, int PER, typename TV>
-__device__ __forceinline__ void dstage1(const DenseSmem& d, const CsrView& R, const CsrView& A,
-                                        int rb, int rlen, int cb, int ce, int nw) {
+//
+// PAGED: [cb, ce) is the whole span, mapped to pages of 2^sh columns.  False
+// when the pages ran out (the slice is to be cleared then).
+template <bool NUM, int PER, bool PAGED, typename TV>
+__device__ __forceinline__ bool dstage1(const DenseSmem& d, const CsrView& R, const CsrView& A,
+                                        int rb, int rlen, int cb, int ce, int nw, int sh) {
     const int tid = threadIdx.x;
     const int nt = nw * 32;
     const int lane = tid & 31;
@@ -468,6 +514,7 @@ __device__ __forceinline__ void dstage1(const DenseSmem& d, const CsrView& R, co
         __syncthreads();
         if (wid >= nw) {
             __syncthreads();
+            if (PAGED && *d.s_pages > kDSpan >> sh) return false;
             continue;
         }
         // pc / pvv[q][j]: the product of entry tid + j * nt of the right row
@@ -514,8 +561,9 @@ __device__ __forceinline__ void dstage1(const DenseSmem& d, const CsrView& R, co
                     const double s = NUM ? st_s[t] : 0.0;
 #pragma unroll
                     for (int j = 0; j < PER; ++j) {
-                        if (col[j] >= cb && col[j] < ce) {
-                            const int slot = col[j] - cb;
+                        const int slot = PAGED ? (col[j] >= 0 ? dpage_slot(d, col[j], cb, sh) : -1)
+                                               : (col[j] >= cb && col[j] < ce ? col[j] - cb : -1);
+                        if (slot >= 0) {
                             if (!d.touched[slot]) {
                                 d.touched[slot] = 1;
                                 d.ftq[slot] = fo + tid + j * nt;
@@ -527,8 +575,9 @@ __device__ __forceinline__ void dstage1(const DenseSmem& d, const CsrView& R, co
                     const int ab_t = st_ab[t], ae_t = st_ae[t];
                     for (int e = ab_t + tid + PER * nt; e < ae_t; e += nt) {
                         const int c2 = __ldg(A.ci + e);
-                        if (c2 >= cb && c2 < ce) {
-                            const int slot = c2 - cb;
+                        const int slot = PAGED ? dpage_slot(d, c2, cb, sh)
+                                               : (c2 >= cb && c2 < ce ? c2 - cb : -1);
+                        if (slot >= 0) {
                             if (!d.touched[slot]) {
                                 d.touched[slot] = 1;
                                 d.ftq[slot] = fo + (e - ab_t);
@@ -542,7 +591,9 @@ __device__ __forceinline__ void dstage1(const DenseSmem& d, const CsrView& R, co
             }
         }
         __syncthreads();
+        if (PAGED && *d.s_pages > kDSpan >> sh) return false;
     }
+    return true;
 }
 
 // One output row of C = R*A*P (row `row` of R) by the whole CTA.  `finish`
@@ -588,33 +639,62 @@ __device__ __forceinline__ void dense_row(const DenseSmem& d, const CsrView& R, 
     const int lo1 = *d.s_lo, hi1 = *d.s_hi;
     const int amax1 = *d.s_cnt;
     const int nw1 = min(kDWarps, max(1, (amax1 + 31) >> 5));
-    for (long long c0 = lo1; c0 <= hi1; c0 += kDSpan) {
+    // List a column of the slice (value and first touch) and clear it.
+    auto list = [&](int slot, int col, bool hit) {
+        const unsigned b = __ballot_sync(kFull, hit);
+        int pos0 = 0;
+        if (lane == 0 && b) pos0 = atomicAdd(d.s_n1, __popc(b));
+        pos0 = __shfl_sync(kFull, pos0, 0);
+        if (hit) {
+            const int pos = pos0 + __popc(b & lt);
+            if (pos < kDList) {
+                d.lkey[pos] = col;
+                d.lq[pos] = d.ftq[slot];
+                if (NUM) d.lval[pos] = d.acc[slot];
+            }
+            d.touched[slot] = 0;
+            if (NUM) d.acc[slot] = 0.0;
+        }
+    };
+    const long long span1 = static_cast<long long>(hi1) - lo1 + 1;
+    bool paged = span1 > kDSpan;
+    if (paged) {
+        int sh = 3;
+        while (span1 > static_cast<long long>(kDPages) << sh) ++sh;
+        paged = sh <= 6;
+        if (paged) {
+            for (int i = threadIdx.x; i < kDPages; i += blockDim.x) d.pt[i] = -1;
+            if (threadIdx.x == 0) *d.s_pages = 0;
+            __syncthreads();
+            paged = amax1 > 32 * kDWarps
+                        ? dstage1<NUM, 2, true, TV>(d, R, A, rb, rlen, lo1, hi1 + 1, nw1, sh)
+                        : dstage1<NUM, 1, true, TV>(d, R, A, rb, rlen, lo1, hi1 + 1, nw1, sh);
+            const int slots = min(*d.s_pages, kDSpan >> sh) << sh;
+            if (paged) {
+                for (int s0 = 32 * wid; s0 < slots; s0 += 32 * kDWarps) {
+                    const int slot = s0 + lane;
+                    const bool hit = slot < slots && d.touched[slot];
+                    list(slot, hit ? d.pcol[slot >> sh] + (slot & ((1 << sh) - 1)) : 0, hit);
+                }
+            } else {   // too many pages: clear the slice and walk it in chunks
+                for (int s0 = threadIdx.x; s0 < kDSpan; s0 += blockDim.x) {
+                    d.touched[s0] = 0;
+                    if (NUM) d.acc[s0] = 0.0;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (long long c0 = lo1; !paged && c0 <= hi1; c0 += kDSpan) {
         const int cb = static_cast<int>(c0);
         const int ce = static_cast<int>(min(static_cast<long long>(hi1) + 1, c0 + kDSpan));
         if (amax1 > 32 * kDWarps)
-            dstage1<NUM, 2, TV>(d, R, A, rb, rlen, cb, ce, nw1);
+            dstage1<NUM, 2, false, TV>(d, R, A, rb, rlen, cb, ce, nw1, 0);
         else
-            dstage1<NUM, 1, TV>(d, R, A, rb, rlen, cb, ce, nw1);
-        // List the slice's touched columns (value and first touch) and
-        // clear them.
+            dstage1<NUM, 1, false, TV>(d, R, A, rb, rlen, cb, ce, nw1, 0);
         for (int s0 = cb + 32 * wid; s0 < ce; s0 += 32 * kDWarps) {
             const int col = s0 + lane;
-            const bool hit = col < ce && d.touched[col - cb];
-            const unsigned b = __ballot_sync(kFull, hit);
-            int pos0 = 0;
-            if (lane == 0 && b) pos0 = atomicAdd(d.s_n1, __popc(b));
-            pos0 = __shfl_sync(kFull, pos0, 0);
-            if (hit) {
-                const int slot = col - cb;
-                const int pos = pos0 + __popc(b & lt);
-                if (pos < kDList) {
-                    d.lkey[pos] = col;
-                    d.lq[pos] = d.ftq[slot];
-                    if (NUM) d.lval[pos] = d.acc[slot];
-                }
-                d.touched[slot] = 0;
-                if (NUM) d.acc[slot] = 0.0;
-            }
+            list(col - cb, col, col < ce && d.touched[col - cb]);
         }
         __syncthreads();
     }
@@ -739,9 +819,9 @@ template <int MODE, typename TV, typename TO>
 __global__ void __launch_bounds__(kDWarps * 32, SP3MM_DENSE_MINB)
     k_direct_dense(DirectRowArgs a, RowParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int s_n1, s_lo, s_hi, s_cnt[kDWarps];
+    __shared__ int s_n1, s_lo, s_hi, s_cnt[kDWarps], s_pages;
     __shared__ long long s_base;
-    const DenseSmem d = dense_smem(smem, &s_n1, &s_lo, &s_hi, s_cnt, &s_base);
+    const DenseSmem d = dense_smem(smem, &s_n1, &s_lo, &s_hi, s_cnt, &s_pages, &s_base);
     dense_clear(d);
     int* oc = MODE == kNumBook ? p.ub_ci : p.c_ci;
     TO* ov = static_cast<TO*>(MODE == kNumBook ? p.ub_v : p.c_v);

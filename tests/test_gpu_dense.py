@@ -161,3 +161,35 @@ def test_wide_operands_run_the_small_configuration_then_the_default(orc):
         ctx.set_tuning(0, -1, -1)
         for m in d:
             m.free()
+
+
+@pytest.mark.parametrize("n_cols,runs,run", [
+    (9000, 24, 40),      # a page table of 8-column pages, runs of several pages
+    (30000, 60, 9),      # runs that just exceed a page, at any offset
+    (40000, 900, 1),     # a page per column: more pages than the slice holds
+    (250000, 40, 70),    # the widest page (64 columns) of the widest span
+    (300000, 20, 30),    # a span beyond the page table: chunks
+])
+def test_paged_slices(orc, n_cols, runs, run):
+    # R*A rows of a few thousand columns at most in runs spread over more
+    # columns than a slice: the slice is paged; with too many pages, or too
+    # wide a span, the row walks its span in chunks.
+    import scipy.sparse as sp
+    rng = np.random.default_rng(runs)
+    pool = [np.arange(s, min(s + run, n_cols)) for s in
+            np.concatenate([[0, n_cols - run], rng.integers(0, n_cols, runs)])]
+    rows = []
+    for i in range(300):
+        take = [0, 1] if i == 0 else rng.choice(len(pool), rng.integers(1, 6), replace=False)
+        c = np.unique(np.concatenate([pool[j] for j in take]))
+        rows.append(np.sort(rng.choice(c, rng.integers(1, len(c) + 1), replace=False)))
+    rows[7] = np.zeros(0, np.int64)
+    n = np.array([len(r) for r in rows])
+    Am = sp.csr_matrix((rng.uniform(-1.5, 1.5, n.sum()), np.concatenate(rows),
+                        np.concatenate([[0], np.cumsum(n)])), shape=(300, n_cols))
+    A = pb.CSR(Am.indptr, Am.indices, Am.data, Am.shape)
+    R = pb.random_sparse(12, 300, 0.6, seed=41, empty_rows=0.1)
+    P = pb.random_sparse(n_cols, 200, 4.0 / 200, seed=42)
+    with S.Context() as ctx:
+        _direct_all_ways(ctx, orc, R, A, P, ("paged", n_cols, runs, run))
+        _direct_all_ways(ctx, orc, R, A, P, ("paged f32", n_cols, runs, run), vt=S.F32)

@@ -250,14 +250,19 @@ struct RowRunner {
     }
 
     // Entries of booking space: SpMM results may hold several times their
-    // operands' nonzeros, Galerkin products (and the batches, which book by
-    // the same rule) a third of theirs.  Eight times those of a 128^3
-    // hierarchy's first product was 2.8 GB allocated and freed per build, and
-    // a program that holds its last hierarchy while it builds the next made
-    // the pool remap it: 30 ms a build against 24.
+    // operands' nonzeros, direct products less than them; Galerkin products
+    // (R as P^T: its rows are P's columns, with as many entries) hold a third
+    // or less.  Eight times those of a 128^3 hierarchy's first product was
+    // 2.8 GB allocated and freed per build, and a program that holds its last
+    // hierarchy while it builds the next made the pool remap it: 30 ms a build.
+    // Twice: 18-29 ms with stalls up to 300; once: 18.1-20.5, as without
+    // the held one (18.4).
     unsigned long long booked_entries() const {
-        return direct ? 2ULL * static_cast<unsigned long long>(da.R.nnz + da.A.nnz + da.P.nnz)
-                      : 8ULL * static_cast<unsigned long long>(pa.A.nnz + pa.B.nnz);
+        if (!direct) return 8ULL * static_cast<unsigned long long>(pa.A.nnz + pa.B.nnz);
+        const unsigned long long all =
+            static_cast<unsigned long long>(da.R.nnz + da.A.nnz + da.P.nnz);
+        const bool galerkin = da.R.M == da.P.N && da.R.nnz == da.P.nnz;
+        return galerkin ? all : 2 * all;
     }
 
     int launch(RowParams p, int G, DevBuf& gtab) {

@@ -140,6 +140,18 @@ def test_booking_space_overflows(orc, a_cols):
     _check(orc, [R, A, P])
 
 
+@pytest.mark.parametrize("a_cols", [1, 600])
+def test_galerkin_booking_space_overflows(orc, a_cols):
+    # The same for operands that look like R = P^T (as many rows as P has
+    # columns, as many entries), whose space is the operands' nonzeros once.
+    rng = np.random.default_rng(9)
+    R = _rows(rng, 1100, 1, 1, 1)
+    A = _rows(rng, 1, a_cols, a_cols, a_cols)
+    ptr = np.unique(np.linspace(0, 1100, a_cols + 1).astype(np.int64))
+    P = S.CSR(ptr, np.arange(1100, dtype=np.int64), rng.uniform(-1.0, 1.0, 1100), (a_cols, 1100))
+    _check(orc, [R, A, P])
+
+
 @pytest.mark.parametrize("vt", [S.F64, S.F32])
 @pytest.mark.parametrize("fl", [S.UB, S.SYMBNUM])
 def test_batches(fl, vt):

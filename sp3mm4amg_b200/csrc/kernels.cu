@@ -14,8 +14,10 @@
 
 #include <atomic>
 #include <climits>
+#include <exception>
 
 #include "kernels.cuh"
+#include "smem_limit.h"
 #include "sp3mm_internal.cuh"
 
 namespace sp3mm {
@@ -23,6 +25,28 @@ namespace sp3mm {
 static std::atomic<uint64_t> g_launches{0};
 uint64_t launch_count() { return g_launches.load(); }
 void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+
+namespace {
+struct SetSmemLimit {
+    int operator()(const void* f, size_t bytes) const {
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(bytes));
+    }
+};
+}  // namespace
+
+cudaError_t raise_smem_limit(const void* f, size_t bytes) {
+    // Never destroyed: a thread may launch while the process exits.
+    static SmemLimits<SetSmemLimit>* limits = new SmemLimits<SetSmemLimit>(SetSmemLimit{});
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    try {
+        return static_cast<cudaError_t>(limits->need(device, f, bytes));
+    } catch (const std::exception&) {   // out of host memory
+        return cudaErrorMemoryAllocation;
+    }
+}
 
 __device__ __forceinline__ double load_val(const void* p, int vt, long long i) {
     if (vt == SP3MM_F32) return static_cast<double>(__ldg(static_cast<const float*>(p) + i));

@@ -223,6 +223,9 @@ void launch_colparts_ub(const CsrView& A, int gridCols, const long long* bColOff
                         long long* out, unsigned long long* total, cudaStream_t st);
 
 void note_launch();
+// Make the current device's dynamic shared-memory limit of kernel `f` at least
+// `bytes` (smem_limit.h: it never shrinks, whichever threads launch f).
+cudaError_t raise_smem_limit(const void* f, size_t bytes);
 uint64_t launch_count();
 
 }  // namespace sp3mm

@@ -572,13 +572,12 @@ __global__ void __launch_bounds__(256) k_pair_rows(PairRowArgs a, RowParams p) {
     }
 }
 
-// Launch one instantiation (sets the dynamic shared-memory limit first).
+// Launch one instantiation (raises the dynamic shared-memory limit first).
 template <typename K, typename Args>
 cudaError_t launch_row_kernel(K k, const Args& a, const RowParams& p, const RowGeom& geo,
                               cudaStream_t st) {
     if (geo.smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(geo.smem));
+        const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), geo.smem);
         if (e != cudaSuccess) return e;
     }
     k<<<geo.grid, geo.block, geo.smem, st>>>(a, p);

@@ -40,9 +40,8 @@ template <int U, int MODE, typename TV, typename TO>
 cudaError_t batch_launch(int ctas, size_t smem, cudaStream_t st, const BItem* items,
                          const int4* chunks, const BatchRowParams& p, const BatchReplay& r) {
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(
-            k_batch_replay<U, MODE, TV, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            static_cast<int>(smem));
+        const cudaError_t e = raise_smem_limit(
+            reinterpret_cast<const void*>(&k_batch_replay<U, MODE, TV, TO>), smem);
         if (e != cudaSuccess) return e;
     }
     k_batch_replay<U, MODE, TV, TO><<<ctas, 32 * kReplayWarps, smem, st>>>(items, chunks, p, r);

@@ -691,8 +691,8 @@ int batch_plan(sp3mm_batch* b) {
     DevBuf ub_ci, ub_v, row_off, cursor;
     if (b->flavour == SP3MM_UB && rows > 0) {
         // One numeric pass: every row books its exact length from one
-        // cursor, in space bounded by twice the operands' nonzeros (and a
-        // replaying warp's handout) and by half the free memory (a batch that
+        // cursor, in space bounded by twice the operands' nonzeros (and each
+        // replaying warp's last handout) and by half the free memory (a batch that
         // overflows it is planned symbolically instead).  Galerkin products
         // and their A*P0 steps write well under their operands' nonzeros;
         // reserving more made the pool map tens of GB for a batch of large

@@ -836,7 +836,7 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
         if (cap * eb > (size_t(1) << 30) && pool_idle_bytes(ctx) < cap * eb)
             cap = std::min<unsigned long long>(
                 cap, std::max<unsigned long long>(1ULL << 20, free_device_bytes(ctx) / 2 / eb));
-        if (replay)   // every warp may leave most of its last handout unused
+        if (replay)   // a warp may leave most of its last handout (at most kReplayBook) unused
             cap += static_cast<unsigned long long>(geometry(kNumBook).grid) * kReplayWarps *
                    kReplayBook;
         TRY(ub_ci.alloc(ctx, sizeof(int) * cap));

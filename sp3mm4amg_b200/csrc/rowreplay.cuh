@@ -395,14 +395,19 @@ __device__ __forceinline__ double2 replay_sums(const ReplayStage& st, const Repl
     return x;
 }
 
-// Space in the booked output, taken kReplayBook entries at a time so that a
-// warp seldom waits for the cursor.
+// Space in the booked output, taken about kReplayBook entries at a time so that
+// a warp seldom waits for the cursor.
 struct ReplayBook {
     unsigned long long at = 0, end = 0;
-    // n entries; -1 when the space is exhausted (flagged).
+    // n entries (a CTA's rows all have the template's); -1 when the space is
+    // exhausted (flagged).  Whole rows are taken, so that only a warp's last
+    // handout, of at most kReplayBook entries, is not used up: with 512 for
+    // rows of 86, every handout lost 82, and 200,000 rows whose space was their
+    // products (17.2 M) overflowed it and were formed again with exact sizes.
     __device__ __forceinline__ long long take(const RowParams& p, int n) {
         if (end - at < static_cast<unsigned long long>(n)) {
-            const unsigned long long want = n > kReplayBook ? n : kReplayBook;
+            const unsigned long long want =
+                n < kReplayBook ? kReplayBook / n * static_cast<unsigned long long>(n) : n;
             unsigned long long b = 0;
             if ((threadIdx.x & 31) == 0) b = atomicAdd(p.cursor, want);
             at = __shfl_sync(kFull, b, 0);

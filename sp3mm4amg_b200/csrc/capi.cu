@@ -249,20 +249,28 @@ struct RowRunner {
         return avg >= 0.75 * (1 << lg) ? lg : -1;
     }
 
-    // Entries of booking space: SpMM results may hold several times their
-    // operands' nonzeros, direct products less than them; Galerkin products
-    // (R as P^T: its rows are P's columns, with as many entries) hold a third
-    // or less.  Eight times those of a 128^3 hierarchy's first product was
-    // 2.8 GB allocated and freed per build, and a program that holds its last
-    // hierarchy while it builds the next made the pool remap it: 30 ms a build.
-    // Twice: 18-29 ms with stalls up to 300; once: 18.1-20.5, as without
-    // the held one (18.4).
+    // The direct product's P is one smoothing step of an aggregation of A, and
+    // R its transpose (a hierarchy's own level).
+    bool smoothed = false;
+
+    // Entries of booking space (a product that overflows it is redone with
+    // exact sizes): results may hold several times their operands' nonzeros
+    // (A*A*A of a 7-point operator 3 times, R*A*P over a random graph 8), and
+    // eight times them costs nothing but the space.  A hierarchy's levels are
+    // the exception: for the first product of a 128^3 one that is 2.8 GB
+    // allocated and freed per build, and a program that holds its last
+    // hierarchy while it builds the next made the pool remap it: 30 ms a
+    // build, against 18.1-20.5 with the operands' nonzeros once, and 18.4
+    // without the held one.  Once is enough where the aggregates' points share
+    // neighbours, that is where P holds fewer entries than A: at most 3/4 of
+    // them on grids and narrow bands, whose products hold at most 0.47 of the
+    // operands' nonzeros; 0.96-1.0 on kNN and random graphs and wide bands,
+    // whose products hold 2.3 to 10.6 times.
     unsigned long long booked_entries() const {
         if (!direct) return 8ULL * static_cast<unsigned long long>(pa.A.nnz + pa.B.nnz);
         const unsigned long long all =
             static_cast<unsigned long long>(da.R.nnz + da.A.nnz + da.P.nnz);
-        const bool galerkin = da.R.M == da.P.N && da.R.nnz == da.P.nnz;
-        return galerkin ? all : 2 * all;
+        return smoothed && 4 * da.P.nnz <= 3 * da.A.nnz ? all : 8 * all;
     }
 
     int launch(RowParams p, int G, DevBuf& gtab) {
@@ -934,7 +942,7 @@ int spmm_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flav
 
 // C = R*A*P, direct (row forwarding).
 int direct_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const sp3mm_dcsr& P,
-                int flavour, int out_vt, sp3mm_dcsr* C) {
+                int flavour, int out_vt, bool smoothed, sp3mm_dcsr* C) {
     if (R.N != A.M || A.N != P.M)
         return set_error(ctx, SP3MM_EINVAL, "inner dimensions differ");
     if (R.val_type != A.val_type || A.val_type != P.val_type)
@@ -951,7 +959,8 @@ int direct_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const 
     TRY(known_max_row(ctx, A, &amax));
     ReplayCaps caps;
     if (plain_tuning(ctx) && bounded_rows(true, R.max_row, amax, A.N, pmax, P.N, &caps)) {
-        RowRunner rr{ctx, true, kSymb, DirectRowArgs{view(R), view(A), view(P)}, {}, amax, pmax};
+        RowRunner rr{ctx, true, kSymb, DirectRowArgs{view(R), view(A), view(P)}, {}, amax, pmax,
+                     smoothed};
         const long long s1 = std::min<long long>(static_cast<long long>(R.max_row) * amax, A.N);
         const long long s2 = std::min<long long>(s1 * pmax, P.N);
         return product_bounded(ctx, rr, M, P.N, flavour, out_vt, caps, s1, s2,
@@ -967,7 +976,8 @@ int direct_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const 
         launch_direct_bounds(view(R), view(A), pmax, need.as<int>(), &dc->total, st,
                              need_opt.as<int>(), d1);
     });
-    RowRunner rr{ctx, true, kSymb, DirectRowArgs{view(R), view(A), view(P)}, {}, amax, pmax};
+    RowRunner rr{ctx, true, kSymb, DirectRowArgs{view(R), view(A), view(P)}, {}, amax, pmax,
+                     smoothed};
     return product_rows(ctx, rr, M, P.N, flavour, out_vt, need, dc, G, d1, d2, A.N, P.N,
                         static_cast<double>(pmax), C, need_opt.as<int>());
 }
@@ -983,8 +993,8 @@ void free_dcsr_arrays(sp3mm_ctx* ctx, sp3mm_dcsr* m) {
 }
 
 int rap_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const sp3mm_dcsr& P,
-             int variant, int flavour, int out_vt, sp3mm_dcsr* C) {
-    if (variant == SP3MM_DIRECT) return direct_impl(ctx, R, A, P, flavour, out_vt, C);
+             int variant, int flavour, int out_vt, sp3mm_dcsr* C, bool smoothed = false) {
+    if (variant == SP3MM_DIRECT) return direct_impl(ctx, R, A, P, flavour, out_vt, smoothed, C);
     sp3mm_dcsr T{};
     int rc;
     // The intermediate is stored in the operands' value type (FP64 operands:
@@ -1593,6 +1603,13 @@ spmat* pair_driver(spmat* R, spmat* AC, spmat* P, CONFIG* cfg, SPMM_INTERF spmm,
 namespace sp3mm {
 int report_error(sp3mm_ctx* ctx, int code, const char* msg) {
     return set_error(ctx, code, "%s", msg);
+}
+int rap_smoothed(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const sp3mm_dcsr& P,
+                 int variant, int flavour, int out_vt, sp3mm_dcsr* C) {
+    TRY(check_dcsr(ctx, &R, "R"));
+    TRY(check_dcsr(ctx, &A, "A"));
+    TRY(check_dcsr(ctx, &P, "P"));
+    return rap_impl(ctx, R, A, P, variant, flavour, out_vt, C, true);
 }
 }  // namespace sp3mm
 

@@ -278,7 +278,7 @@ int sp3mm_hierarchy_build(sp3mm_ctx* ctx, const sp3mm_dcsr* A0, const int32_t* d
         // The product needs one storage type: R and P follow A's.
         if (rc == SP3MM_OK && P.val_type != A.val_type)
             rc = fail(ctx, SP3MM_EINVAL, "hierarchy_build: level value types differ");
-        if (rc == SP3MM_OK) rc = sp3mm_rap(ctx, &R, &A, &P, variant, flavour, avt, &Ac);
+        if (rc == SP3MM_OK) rc = rap_smoothed(ctx, R, A, P, variant, flavour, avt, &Ac);
         if (rc != SP3MM_OK) {
             sp3mm_dcsr_free(ctx, &P);
             sp3mm_dcsr_free(ctx, &R);

@@ -48,4 +48,9 @@ int hierarchy_step(sp3mm_ctx* ctx, const std::vector<sp3mm_hierarchy*>& hs);
 constexpr int kAggProductRow = 32;
 int agg_product(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const int* agg, int nc, sp3mm_dcsr* AP0);
 
+// sp3mm_rap of a level's own operands (P one smoothing step of an aggregation
+// of A, R its transpose): its direct product may book less space.
+int rap_smoothed(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const sp3mm_dcsr& P,
+                 int variant, int flavour, int out_vt, sp3mm_dcsr* C);
+
 }  // namespace sp3mm

@@ -93,3 +93,73 @@ def test_batch_overflows_after_replayed_rows(orc):
         for x in d:
             for m in x:
                 m.free()
+
+
+def _cubes():
+    import scipy.sparse as sp
+    from sp3mm4amg_b200 import problems as pb
+    rng = np.random.default_rng(3)
+
+    def rand(M, N, lo, hi):
+        n = rng.integers(lo, hi + 1, M)
+        row = np.repeat(np.arange(M), n)
+        m = sp.csr_matrix((rng.uniform(-1, 1, len(row)), (row, rng.integers(0, N, len(row)))),
+                          shape=(M, N))
+        m.sum_duplicates()
+        m.sort_indices()
+        return S.CSR(m.indptr.astype(np.int64), m.indices.astype(np.int64), m.data, m.shape)
+
+    box, grid = pb.poisson3d(44), pb.poisson2d(320)
+    A, P = rand(60000, 60000, 6, 8), rand(60000, 30000, 2, 4)
+    return {"7-point cubed": [box] * 3, "5-point cubed": [grid] * 3,
+            "random Galerkin": [P.transpose(), A, P],
+            "random bounded": [rand(60000, 60000, 3, 6), rand(60000, 60000, 5, 15),
+                               rand(60000, 30000, 1, 3)]}
+
+
+@pytest.mark.parametrize("which", ["7-point cubed", "5-point cubed", "random Galerkin",
+                                   "random bounded"])
+def test_results_of_several_times_the_operands(orc, which):
+    # Results of 1.6 to 7 times their operands' nonzeros (and more than 2^20),
+    # also where R and P have the shapes and lengths of transposes.
+    ops = _cubes()[which]
+    want = orc.sp3mm_direct(*ops)
+    assert want.nnz > 1.6 * sum(m.nnz for m in ops) and want.nnz > 1 << 20
+    with S.Context() as ctx:
+        d = [ctx.upload(m) for m in ops]
+        C, labels = _passes(ctx, lambda: ctx.rap(*d, S.DIRECT, S.UB))
+        assert _booked_once(labels), labels
+        _same(C, want, which)
+        C.free()
+        for m in d:
+            m.free()
+
+
+@pytest.mark.parametrize("kind", ["grid", "wide band"])
+def test_hierarchies_book_enough(kind):
+    # One level of a grid (less space booked) and of a band whose product holds
+    # over twice its operands' nonzeros.
+    from sp3mm4amg_b200 import problems as pb
+    rng = np.random.default_rng(4)
+    if kind == "grid":
+        dims = (90, 80, 70)
+        A = pb.poisson3d(*dims)
+    else:
+        import scipy.sparse as sp
+        n = 100000
+        dims = (n,)
+        row = np.repeat(np.arange(n), 4)
+        col = np.clip(row + rng.integers(-60, 61, 4 * n), 0, n - 1)
+        m = sp.csr_matrix((rng.uniform(-1, 1, 4 * n), (row, col)), shape=(n, n))
+        m = (m + m.T + 10 * sp.eye(n)).tocsr()
+        m.sort_indices()
+        A = S.CSR(m.indptr.astype(np.int64), m.indices.astype(np.int64), m.data, m.shape)
+    with S.Context() as ctx:
+        d = ctx.upload(A)
+        ctx.set_profiling(True)
+        h = ctx.hierarchy(d, dims, max_levels=2)
+        labels = set(ctx.profile())
+        ctx.set_profiling(False)
+        assert _booked_once({x for x in labels if x.startswith("direct.")}), labels
+        h.free()
+        d.free()

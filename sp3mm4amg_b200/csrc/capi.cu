@@ -502,6 +502,15 @@ bool bounded_rows(bool direct, int k1, int l1, int n1, int l2, int n2, ReplayCap
     return true;
 }
 
+// Most entries of a result of M rows of at most `row` entries, each of the left
+// operand's nnz entries giving at most `per` of them (one long row among short
+// ones: a million rows of R with one entry and one row with 64 booked 960 MB
+// where the operands allow 96).
+unsigned long long out_bound(int M, long long row, long long nnz, long long per) {
+    return std::min(static_cast<unsigned long long>(M) * static_cast<unsigned long long>(row),
+                    static_cast<unsigned long long>(nnz) * static_cast<unsigned long long>(per));
+}
+
 int finish_matrix(sp3mm_dcsr* C, DevBuf& rp, DevBuf& ci, DevBuf& v) {
     C->row_ptr = static_cast<int*>(rp.detach());
     C->col = static_cast<int*>(ci.detach());
@@ -925,7 +934,7 @@ int spmm_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flav
         RowRunner rr{ctx, false, kSymb, {}, PairRowArgs{view(A), view(B)}, -1, B.max_row};
         return product_bounded(ctx, rr, M, B.N, flavour, out_vt, caps,
                                std::min<long long>(caps.np1, B.N), 0,
-                               static_cast<unsigned long long>(M) * caps.np1, C);
+                               out_bound(M, caps.np1, A.nnz, B.max_row), C);
     }
     const int d1 = ctx->tune_d1 >= 0 ? ctx->tune_d1 : 2;
     DevBuf cnt_buf, need;
@@ -964,7 +973,7 @@ int direct_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const 
         const long long s1 = std::min<long long>(static_cast<long long>(R.max_row) * amax, A.N);
         const long long s2 = std::min<long long>(s1 * pmax, P.N);
         return product_bounded(ctx, rr, M, P.N, flavour, out_vt, caps, s1, s2,
-                               static_cast<unsigned long long>(M) * s2, C);
+                               out_bound(M, s2, R.nnz, static_cast<long long>(amax) * pmax), C);
     }
     DevBuf cnt_buf, need, need_opt;
     TRY(cnt_buf.alloc(ctx, sizeof(Counters)));

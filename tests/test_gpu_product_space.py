@@ -163,3 +163,52 @@ def test_hierarchies_book_enough(kind):
         assert _booked_once({x for x in labels if x.startswith("direct.")}), labels
         h.free()
         d.free()
+
+
+def _pool_peak(ctx, f):
+    """Most bytes in use in the device's memory pool during f(), above those
+    in use before."""
+    from cuda.bindings import driver, runtime as rt
+
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r
+        return r[1] if len(r) > 1 else None
+
+    attr = rt.cudaMemPoolAttr
+    ctx.sync()
+    pool = ok(rt.cudaDeviceGetDefaultMemPool(0))
+    ok(rt.cudaMemPoolSetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh, driver.cuuint64_t(0)))
+    before = int(ok(rt.cudaMemPoolGetAttribute(pool, attr.cudaMemPoolAttrUsedMemCurrent)))
+    f()
+    ctx.sync()
+    return int(ok(rt.cudaMemPoolGetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh))) - before
+
+
+@pytest.mark.parametrize("variant", [S.DIRECT, S.PAIR])
+def test_space_of_uneven_rows(variant):
+    # One left row of 64 entries among 600,000 of one: the rows' bound (64
+    # times 8 products) is 60 times what the operands allow.  The space stays
+    # within the call's memory estimate.
+    rng = np.random.default_rng(5)
+    M, N = 600000, 500000
+    n = np.ones(M, np.int64)
+    n[M // 2] = 64
+    ptr = np.concatenate([[0], np.cumsum(n)])
+    R = S.CSR(ptr, np.concatenate([np.sort(rng.choice(N, 64, replace=False)) if k > 1 else
+                                   rng.integers(0, N, 1) for k in n]).astype(np.int64),
+              rng.uniform(-1, 1, int(ptr[-1])), (M, N))
+    A = S.CSR(np.arange(N + 1, dtype=np.int64) * 8,
+              (np.arange(N)[:, None] + np.arange(8)).ravel().astype(np.int64),
+              rng.uniform(-1, 1, 8 * N), (N, N + 8))
+    P = S.CSR(np.arange(N + 9, dtype=np.int64), np.arange(N + 8, dtype=np.int64),
+              np.ones(N + 8), (N + 8, N + 8))
+    with S.Context() as ctx:
+        d = [ctx.upload(m) for m in (R, A, P)]
+        got = []
+        peak = _pool_peak(ctx, lambda: got.append(ctx.rap(*d, variant, S.UB)))
+        assert peak <= ctx.rap_memory_estimate(*d, variant, S.UB), peak
+        # (its result holds 8 entries a row: 96 bytes, and as many booked)
+        assert got[0].nnz > 7 * M
+        got[0].free()
+        for m in d:
+            m.free()

@@ -320,22 +320,42 @@ __global__ void k_col_counts(long long nnz, const int* ci, int* counts) {
 }
 
 // 2^lg lanes per row of A (its mean length: a warp per row of the four
-// entries of a fine prolongator took 0.41 ms at 128^3, four lanes 0.09).
+// entries of a fine prolongator took 0.41 ms at 128^3, four lanes 0.09), and
+// the whole warp for a row of more than kScatterLong times its lanes (a row of
+// 200,000 entries among 500,000 of two: 19.6 ms on two lanes, 3.4 on a warp).
+constexpr int kScatterLong = 8;
 __global__ void __launch_bounds__(256) k_transpose_scatter(CsrView A, int lg, const int* t_rp,
-                                                            int* cursor, int* t_ci, void* t_v) {
-    const int sub = threadIdx.x & ((1 << lg) - 1);
-    const long long groups = (static_cast<long long>(gridDim.x) * blockDim.x) >> lg;
-    for (long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> lg; row < A.M;
-         row += groups) {
-        const int b = A.rp[row], e = A.rp[row + 1];
-        for (int j = b + sub; j < e; j += 1 << lg) {
+                                                             int* cursor, int* t_ci, void* t_v) {
+    const int lane = threadIdx.x & 31;
+    const int sub = lane & ((1 << lg) - 1);
+    auto scatter = [&](int row, int b, int e, int step) {
+        for (int j = b; j < e; j += step) {
             const int c = A.ci[j];
             const int pos = t_rp[c] + atomicAdd(cursor + c, 1);
-            t_ci[pos] = static_cast<int>(row);
+            t_ci[pos] = row;
             if (A.vtype == SP3MM_F32)
                 static_cast<float*>(t_v)[pos] = static_cast<const float*>(A.v)[j];
             else
                 static_cast<double*>(t_v)[pos] = static_cast<const double*>(A.v)[j];
+        }
+    };
+    const long long groups = (static_cast<long long>(gridDim.x) * blockDim.x) >> lg;
+    // (row - (lane >> lg): the warp's first row, the same for all its lanes)
+    for (long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> lg;
+         row - (lane >> lg) < A.M; row += groups) {
+        int b = 0, e = 0;
+        if (row < A.M) {
+            b = A.rp[row];
+            e = A.rp[row + 1];
+        }
+        const bool big = e - b > kScatterLong << lg;
+        if (!big) scatter(static_cast<int>(row), b + sub, e, 1 << lg);
+        for (unsigned m = __ballot_sync(0xffffffffu, big && sub == 0); m; m &= m - 1) {
+            const int src = __ffs(m) - 1;
+            const int r = __shfl_sync(0xffffffffu, static_cast<int>(row), src);
+            const int rb = __shfl_sync(0xffffffffu, b, src);
+            const int re = __shfl_sync(0xffffffffu, e, src);
+            scatter(r, rb + lane, re, 32);
         }
     }
 }

@@ -1,0 +1,67 @@
+"""Transposes of matrices whose rows differ widely in length: the same result,
+and one long row among short ones takes about what the long row and the short
+ones take apart."""
+import time
+
+import numpy as np
+import pytest
+
+import sp3mm4amg_b200 as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(rng, lengths, N):
+    """Rows of the given numbers of distinct columns, ascending."""
+    cols = [np.sort(rng.choice(N, n, replace=False)) if n > 8 else
+            np.unique(rng.integers(0, N, n)) for n in lengths]
+    ptr = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int64)
+    return S.CSR(ptr, np.concatenate(cols).astype(np.int64), rng.uniform(-1, 1, int(ptr[-1])),
+                 (len(lengths), N))
+
+
+def _times(ctx, A):
+    d = ctx.upload(A)
+    t = []
+    for _ in range(8):
+        ctx.sync()
+        t0 = time.perf_counter()
+        ctx.transpose(d).free()
+        ctx.sync()
+        t.append(time.perf_counter() - t0)
+    d.free()
+    return min(t)
+
+
+@pytest.mark.parametrize("mean", [1, 3, 9, 20])
+def test_long_rows_among_short(mean):
+    # Every number of lanes per row, rows at their limit (8 times the lanes)
+    # and beyond it, several in one warp, the last row among them.
+    rng = np.random.default_rng(mean)
+    n = rng.integers(0, 2 * mean + 1, 3001)
+    lanes = 1 << int(np.ceil(np.log2(mean)))
+    n[[3, 4, 5, 700, 3000]] = [8 * lanes, 8 * lanes + 1, 8 * lanes - 1, 1900, 1500]
+    A = _rows(rng, n, 2000)
+    want = A.transpose()
+    with S.Context() as ctx:
+        d = ctx.upload(A)
+        T = ctx.transpose(d)
+        got = T.download()
+        T.free()
+        d.free()
+    assert np.array_equal(got.indptr, want.indptr)
+    assert np.array_equal(got.indices, want.indices)
+    assert np.array_equal(got.data, want.data)
+
+
+def test_one_long_row_costs_no_more_than_alone():
+    rng = np.random.default_rng(5)
+    short = np.full(200000, 2)
+    both = short.copy()
+    both[777] = 150000
+    with S.Context() as ctx:
+        t_short = _times(ctx, _rows(rng, short, 200000))
+        t_long = _times(ctx, _rows(rng, [150000], 200000))
+        t_both = _times(ctx, _rows(rng, both, 200000))
+    # (on the lanes of its neighbours the long row took six times as long)
+    assert t_both < 2 * (t_short + t_long), (t_short, t_long, t_both)

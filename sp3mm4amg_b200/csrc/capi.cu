@@ -1901,7 +1901,8 @@ int sp3mm_transpose(sp3mm_ctx* ctx, const sp3mm_dcsr* A, sp3mm_dcsr* AT) {
     CK(ctx, cudaMemsetAsync(mr, 0, sizeof(int), st));
     launch_count_max(M, counts, nullptr, mr, st);
     launch_transpose_scatter(view(*A), rp.as<int>(), counts + words, ci.as<int>(), v.p, st);
-    launch_sort_rows(M, rp.as<int>(), ci.as<int>(), v.p, A->val_type, INT_MAX, st, ctx->d_err);
+    launch_sort_rows(M, rp.as<int>(), ci.as<int>(), v.p, A->val_type, static_cast<int>(A->nnz), st,
+                     ctx->d_err);
     CK(ctx, cudaGetLastError());
     unsigned* box = ctx->host_box;
     CK(ctx, cudaMemcpyAsync(box, mr, sizeof(int), cudaMemcpyDeviceToHost, st));

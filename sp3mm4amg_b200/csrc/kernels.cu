@@ -15,6 +15,7 @@
 #include <atomic>
 #include <climits>
 #include <exception>
+#include <type_traits>
 
 #include "kernels.cuh"
 #include "smem_limit.h"
@@ -364,16 +365,103 @@ __global__ void __launch_bounds__(256) k_transpose_scatter(CsrView A, int lg, co
 // every column's rank (the row in shared memory, four columns compared per
 // load).  The coarse levels' restrictions hold rows of 84 to 677 entries: a
 // warp per row with a bitonic network took 1.13 ms over the levels of a 128^3
-// hierarchy, this 0.43.  A column met twice is flagged where err is given.
+// hierarchy, this 0.43.  Ranks take n^2 comparisons: rows past kSortRankRow
+// entries go to a launch of their own (NET), a bitonic network of one size by
+// the CTA (transpose with 1,000 rows of 2,000: 1.28 -> 0.43 ms; both in one
+// kernel made rows of 700 8 % slower).  A column met twice is flagged where err
+// is given.
 constexpr int kSortSmemRow = 2048;
+constexpr int kSortRankRow = kSortSmemRow / 2;
 constexpr int kSortThreads = 128;
 
+// Bitonic network over kSortSmemRow keys.
+__device__ __forceinline__ void sort_network(unsigned long long* key) {
+    for (int k = 2; k <= kSortSmemRow; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            __syncthreads();
+            for (int q = threadIdx.x; q < kSortSmemRow / 2; q += kSortThreads) {
+                const int i = 2 * q - (q & (j - 1));
+                const unsigned long long a = key[i], c = key[i + j];
+                if ((a > c) == ((i & k) == 0)) {
+                    key[i] = c;
+                    key[i + j] = a;
+                }
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// A row of n > kSortRankRow entries from b on: its columns are sorted with
+// their places, then the values fetched from there into the keys' storage
+// (before any is overwritten) and written.
+__device__ __forceinline__ void sort_row_network(unsigned long long* key, int b, int n, int* ci,
+                                                 void* v, int vt, unsigned* err) {
+    static_assert(kSortSmemRow == 2048, "places take 11 bits");
+    for (int i = threadIdx.x; i < kSortSmemRow; i += kSortThreads)
+        key[i] = i < n ? static_cast<unsigned long long>(ci[b + i]) << 11 | i : ~0ULL;
+    sort_network(key);
+    for (int i = threadIdx.x; i < n; i += kSortThreads) {
+        ci[b + i] = static_cast<int>(key[i] >> 11);
+        if (i > 0 && key[i - 1] >> 11 == key[i] >> 11 && err) atomicOr(err, kErrInput);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kSortThreads)
+        key[i] = __double_as_longlong(load_val(v, vt, b + static_cast<int>(key[i] & 2047)));
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kSortThreads)
+        store_val(v, vt, b + i, __longlong_as_double(key[i]));
+    __syncthreads();
+}
+
+// A row of n > 32 entries from b on by ranks.
+__device__ __forceinline__ void sort_row_ranks(int* sk, double* sv, int b, int n, int* ci,
+                                               void* v, int vt, unsigned* err) {
+    constexpr int U = 4;   // columns a thread ranks together
+    for (int i = threadIdx.x; i < n; i += kSortThreads) {
+        sk[i] = ci[b + i];
+        sv[i] = load_val(v, vt, b + i);
+    }
+    if (threadIdx.x < 4) sk[n + threadIdx.x] = INT_MAX;
+    __syncthreads();
+    for (int i0 = threadIdx.x; i0 < n; i0 += U * kSortThreads) {
+        int k[U], lt[U], eq[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * kSortThreads;
+            k[u] = i < n ? sk[i] : -1;
+            lt[u] = eq[u] = 0;
+        }
+        for (int j = 0; j < n; j += 4) {
+            const int4 q = *reinterpret_cast<const int4*>(sk + j);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (u * kSortThreads < n) {
+                    lt[u] += (q.x < k[u]) + (q.y < k[u]) + (q.z < k[u]) + (q.w < k[u]);
+                    eq[u] += (q.x == k[u]) + (q.y == k[u]) + (q.z == k[u]) + (q.w == k[u]);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * kSortThreads;
+            if (i < n) {
+                ci[b + lt[u]] = k[u];
+                store_val(v, vt, b + lt[u], sv[i]);
+                if (eq[u] > 1 && err) atomicOr(err, kErrInput);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+template <bool NET>
 __global__ void __launch_bounds__(kSortThreads) k_sort_rows_cta(int M, int chunk, const int* rp,
                                                                 int* ci, void* v, int vt,
                                                                 unsigned* err) {
-    __shared__ __align__(16) int sk[kSortSmemRow + 4];
-    __shared__ double sv[kSortSmemRow];
-    constexpr int U = 4;   // columns a thread ranks together
+    constexpr int kMin = NET ? kSortRankRow : 32, kMax = NET ? kSortSmemRow : kSortRankRow;
+    __shared__ __align__(16) int sk[NET ? 4 : kMax + 4];
+    __shared__ std::conditional_t<NET, unsigned long long, double> sv[kMax];
     const int lane = threadIdx.x & 31;
     for (long long r0 = blockIdx.x * static_cast<long long>(chunk); r0 < M;
          r0 += gridDim.x * static_cast<long long>(chunk)) {
@@ -383,45 +471,12 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_rows_cta(int M, int chunk
             lb = rp[r0 + lane];
             ln = rp[r0 + lane + 1] - lb;
         }
-        unsigned rows = __ballot_sync(0xffffffffu, ln > 32 && ln <= kSortSmemRow);
+        unsigned rows = __ballot_sync(0xffffffffu, ln > kMin && ln <= kMax);
         for (; rows; rows &= rows - 1) {
             const int b = __shfl_sync(0xffffffffu, lb, __ffs(rows) - 1);
             const int n = __shfl_sync(0xffffffffu, ln, __ffs(rows) - 1);
-            for (int i = threadIdx.x; i < n; i += kSortThreads) {
-                sk[i] = ci[b + i];
-                sv[i] = load_val(v, vt, b + i);
-            }
-            if (threadIdx.x < 4) sk[n + threadIdx.x] = INT_MAX;
-            __syncthreads();
-            for (int i0 = threadIdx.x; i0 < n; i0 += U * kSortThreads) {
-                int k[U], lt[U], eq[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int i = i0 + u * kSortThreads;
-                    k[u] = i < n ? sk[i] : -1;
-                    lt[u] = eq[u] = 0;
-                }
-                for (int j = 0; j < n; j += 4) {
-                    const int4 q = *reinterpret_cast<const int4*>(sk + j);
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        if (u * kSortThreads < n) {
-                            lt[u] += (q.x < k[u]) + (q.y < k[u]) + (q.z < k[u]) + (q.w < k[u]);
-                            eq[u] += (q.x == k[u]) + (q.y == k[u]) + (q.z == k[u]) + (q.w == k[u]);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int i = i0 + u * kSortThreads;
-                    if (i < n) {
-                        ci[b + lt[u]] = k[u];
-                        store_val(v, vt, b + lt[u], sv[i]);
-                        if (eq[u] > 1 && err) atomicOr(err, kErrInput);
-                    }
-                }
-            }
-            __syncthreads();
+            if constexpr (NET) sort_row_network(sv, b, n, ci, v, vt, err);
+            else sort_row_ranks(sk, sv, b, n, ci, v, vt, err);
         }
     }
 }
@@ -658,9 +713,13 @@ void launch_sort_rows(int M, const int* rp, int* ci, void* v, int vt, int max_ro
         // Few rows: one per CTA; many: 32 lengths looked up at once.
         const int ctas = 148 * 8;
         const int chunk = M < ctas ? 1 : M / ctas < 32 ? M / ctas : 32;
-        k_sort_rows_cta<<<grid_for(M, chunk, ctas), kSortThreads, 0, st>>>(M, chunk, rp, ci, v,
-                                                                           vt, err);
+        const int grid = grid_for(M, chunk, ctas);
+        k_sort_rows_cta<false><<<grid, kSortThreads, 0, st>>>(M, chunk, rp, ci, v, vt, err);
         note_launch();
+        if (max_row > kSortRankRow) {
+            k_sort_rows_cta<true><<<grid, kSortThreads, 0, st>>>(M, chunk, rp, ci, v, vt, err);
+            note_launch();
+        }
     }
 }
 

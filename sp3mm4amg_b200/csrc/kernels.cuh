@@ -214,6 +214,7 @@ void launch_validate_i32(int M, int N, const int* rp, const int* ci, int* max_ro
 void launch_col_counts(long long nnz, const int* ci, int* counts, cudaStream_t st);
 void launch_transpose_scatter(const CsrView& A, const int* t_rp, int* cursor, int* t_ci,
                               void* t_v, cudaStream_t st);
+// max_row: no row is longer (the sort kernels skip the rows they do not handle).
 // err (optional): flagged when a row holds a column twice.
 void launch_sort_rows(int M, const int* rp, int* ci, void* v, int vtype, int max_row,
                       cudaStream_t st, unsigned* err = nullptr);

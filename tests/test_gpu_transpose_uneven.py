@@ -65,3 +65,51 @@ def test_one_long_row_costs_no_more_than_alone():
         t_both = _times(ctx, _rows(rng, both, 200000))
     # (on the lanes of its neighbours the long row took six times as long)
     assert t_both < 2 * (t_short + t_long), (t_short, t_long, t_both)
+
+
+@pytest.mark.parametrize("vt", [S.F64, S.F32])
+def test_rows_on_both_sides_of_the_network(vt):
+    rng = np.random.default_rng(6)
+    T = _rows(rng, [1023, 1024, 1025, 1026, 1500, 2046, 2047, 2048, 1025], 5000)
+    if vt == S.F32:
+        T.data[:] = T.data.astype(np.float32)
+    with S.Context() as ctx:
+        d = ctx.upload(T.transpose(), vt)
+        got = ctx.transpose(d).download()
+        d.free()
+    assert np.array_equal(got.indptr, T.indptr)
+    assert np.array_equal(got.indices, T.indices)
+    assert np.array_equal(got.data, T.data)
+
+
+@pytest.mark.parametrize("n", [1025, 2048])
+def test_repeated_column_is_refused(n):
+    # Upload refuses such a row, so the device copy's columns are overwritten.
+    import torch
+    A = _rows(np.random.default_rng(7), [n, n], n + 5).transpose()
+    with S.Context() as ctx:
+        dA = ctx.upload(A)
+        row = int(np.argmax(np.diff(A.indptr)))    # a row of both columns
+
+        class Mem:
+            __cuda_array_interface__ = {"shape": (A.nnz,), "typestr": "<i4",
+                                        "data": (dA.d.col, False), "version": 3}
+        cols = torch.as_tensor(Mem(), device="cuda")
+        ctx.sync()
+        cols[int(A.indptr[row]) + 1] = 0           # column 0 twice in one row
+        torch.cuda.synchronize()
+        with pytest.raises(S.Sp3mmError):
+            ctx.transpose(dA)
+        dA.free()
+
+
+def test_time_does_not_grow_with_the_rows_length():
+    # As many entries in rows of 2,000 as in rows of 1,000 (ranks alone: 1.6
+    # times as long).
+    rng = np.random.default_rng(8)
+    t = {}
+    with S.Context() as ctx:
+        for n in (1000, 2000):
+            A = _rows(rng, [n] * (2000000 // n), 16 * n).transpose()
+            t[n] = _times(ctx, A)
+    assert t[2000] < 1.2 * t[1000], t

@@ -492,6 +492,11 @@ bool plain_tuning(const sp3mm_ctx* ctx) {
 // rows (a bounds launch, two binning launches and a host round trip fewer:
 // the 64x64 product 106 -> 85 us).
 
+// Symbolic retries (and M / 256 of them, what binning M rows takes) from which
+// the exact numeric pass of such a product bins its rows: 300,000 rows of 3 to
+// 6 times 5 to 15 random entries, all but a few retried, 6.1 -> 4.3 ms.
+constexpr int kRebinRetries = 4096;
+
 // Whether rows of at most k1 steps of l1 products (and, direct, of P rows of
 // at most l2) are bounded so, and the replayed kernel's capacities.
 bool bounded_rows(bool direct, int k1, int l1, int n1, int l2, int n2, ReplayCaps* c) {
@@ -836,10 +841,25 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
         return rr.launch(q, 32, gtab);
     };
     TailReads tr{};
+    bool rebin = false;
+    DevBuf row_cnt1;
     if (flavour == SP3MM_SYMBNUM) {
+        if (rr.direct) {
+            TRY(row_cnt1.alloc(ctx, sizeof(int) * (static_cast<size_t>(M) + 1)));
+            p.row_cnt1 = row_cnt1.as<int>();
+        }
         TRY(rows(kSymb));
+        if (replay)
+            CK(ctx, cudaMemcpyAsync(ctx->host_box + 6, n_left, sizeof(int), cudaMemcpyDeviceToHost,
+                                    st));
         TRY(scan_read(ctx, M, row_cnt.as<int>(), rp, &dc->retry_count, &tr));
         if (tr.err) return check_device_err(ctx);
+        // Where many rows outgrew the tables of the bound, the numeric pass
+        // would run them on the retry kernel (about 13 us a thousand rows):
+        // the rows are binned by their counts instead, unless most of them are
+        // replayed.
+        const long long left = replay ? static_cast<int>(ctx->host_box[6]) : M;
+        rebin = !tiny && tr.retry > kRebinRetries + M / 256 && 2 * left > M;
         if (tr.retry > 0) {
             TRY(rr.run_retry(p, tr.retry, retry, s1_max, s2_max));
             TRY(scan_read(ctx, M, row_cnt.as<int>(), rp, nullptr, &tr));
@@ -890,8 +910,22 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
         p.c_rp = rp.as<int>();
         p.c_ci = ci.as<int>();
         p.c_v = v.p;
-        CK(ctx, cudaMemsetAsync(&dc->retry_count, 0, sizeof(int), st));
-        TRY(rows(kNumExact));
+        CK(ctx, cudaMemsetAsync(dc, 0, sizeof(Counters), st));
+        if (rebin) {
+            DevBuf need_cnt;
+            TRY(need_cnt.alloc(ctx, sizeof(int) * (static_cast<size_t>(M) + 1)));
+            prof(ctx, "need", [&] {
+                launch_need_from_counts(M, row_cnt.as<int>(), p.row_cnt1, need_cnt.as<int>(), st);
+            });
+            Bins bins;
+            TRY(bin_rows(ctx, M, need_cnt.as<int>(), 0, 32, dc, nullptr, bins));
+            p.row_cnt1 = nullptr;
+            rr.mode = kNumExact;
+            TRY(rr.run_levels(bins, p, 32, 0, dc, retry));
+        } else {
+            p.row_cnt1 = nullptr;
+            TRY(rows(kNumExact));
+        }
         TRY(read_retry_err(ctx, &dc->retry_count, &tr));
         if (tr.retry > 0 && !tr.err) {
             TRY(rr.run_retry(p, tr.retry, retry, s1_max, s2_max));

@@ -497,6 +497,10 @@ bool plain_tuning(const sp3mm_ctx* ctx) {
 // 6 times 5 to 15 random entries, all but a few retried, 6.1 -> 4.3 ms.
 constexpr int kRebinRetries = 4096;
 
+// Lines of uneven_rows.
+constexpr int kUnevenMinRows = 150000;
+constexpr double kUnevenRatio = 32.0;
+
 // Whether rows of at most k1 steps of l1 products (and, direct, of P rows of
 // at most l2) are bounded so, and the replayed kernel's capacities.
 bool bounded_rows(bool direct, int k1, int l1, int n1, int l2, int n2, ReplayCaps* c) {
@@ -514,6 +518,23 @@ bool bounded_rows(bool direct, int k1, int l1, int n1, int l2, int n2, ReplayCap
 unsigned long long out_bound(int M, long long row, long long nnz, long long per) {
     return std::min(static_cast<unsigned long long>(M) * static_cast<unsigned long long>(row),
                     static_cast<unsigned long long>(nnz) * static_cast<unsigned long long>(per));
+}
+
+// Mean products per row of X*Y.
+double mean_products(const sp3mm_dcsr& X, const sp3mm_dcsr& Y) {
+    return (X.M ? static_cast<double>(X.nnz) / X.M : 0.0) *
+           (Y.M ? static_cast<double>(Y.nnz) / Y.M : 0.0);
+}
+
+// Rows whose bound is far above their mean run with tables far too large for
+// most of them, and from some number of rows on that costs more than bounds and
+// binning do.  One row of 60 among rows of 1 to 3, right rows of 2 to 8 (47
+// times the mean), SpMM and R*A*P in us: 100,000 rows 255 and 473 against 325
+// and 489 binned, 300,000 rows 568 and 931 against 502 and 820, a million 1790
+// and 2641 against 1239 and 2392; one row of 24 (19 times): a million 1013 and
+// 1726 against 1173 and 2067.
+bool uneven_rows(int M, const ReplayCaps& caps, double mean) {
+    return M >= kUnevenMinRows && caps.np1 > kUnevenRatio * mean;
 }
 
 int finish_matrix(sp3mm_dcsr* C, DevBuf& rp, DevBuf& ci, DevBuf& v) {
@@ -959,12 +980,11 @@ int spmm_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flav
     int G = pick_group(ctx, B.M ? static_cast<double>(B.nnz) / B.M : 1.0);
     // Rows of a few products (a hierarchy's A*P0: 7 per row) leave most of
     // a warp idle: 4 lanes a row, 8 rows a warp (128^3 A*P0: 1.76 -> 0.85 ms).
-    const double products = (A.M ? static_cast<double>(A.nnz) / A.M : 0.0) *
-                            (B.M ? static_cast<double>(B.nnz) / B.M : 0.0);
+    const double products = mean_products(A, B);
     if (ctx->tune_G == 0 && products <= 8.0) G = 4;
     ReplayCaps caps;
     if (plain_tuning(ctx) && bounded_rows(false, A.max_row, B.max_row, B.N, 0, 0, &caps) &&
-        (G == 32 || caps.np1 <= kTinyProducts)) {
+        (G == 32 || caps.np1 <= kTinyProducts) && !uneven_rows(M, caps, products)) {
         RowRunner rr{ctx, false, kSymb, {}, PairRowArgs{view(A), view(B)}, -1, B.max_row};
         return product_bounded(ctx, rr, M, B.N, flavour, out_vt, caps,
                                std::min<long long>(caps.np1, B.N), 0,
@@ -1001,7 +1021,8 @@ int direct_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const 
     TRY(known_max_row(ctx, P, &pmax));
     TRY(known_max_row(ctx, A, &amax));
     ReplayCaps caps;
-    if (plain_tuning(ctx) && bounded_rows(true, R.max_row, amax, A.N, pmax, P.N, &caps)) {
+    if (plain_tuning(ctx) && bounded_rows(true, R.max_row, amax, A.N, pmax, P.N, &caps) &&
+        !uneven_rows(M, caps, mean_products(R, A))) {
         RowRunner rr{ctx, true, kSymb, DirectRowArgs{view(R), view(A), view(P)}, {}, amax, pmax,
                      smoothed};
         const long long s1 = std::min<long long>(static_cast<long long>(R.max_row) * amax, A.N);

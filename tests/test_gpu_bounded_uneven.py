@@ -75,3 +75,17 @@ def test_few_rows_past_the_tables_are_not(orc):
     p = pb.stencil_problem(3, (50, 48, 52))
     labels = _labels(orc, [p.R, p.A, p.P])
     assert "bin.levels" not in labels[S.SYMBNUM], labels
+
+
+@pytest.mark.parametrize("M,longest,binned", [(149999, 60, False), (150000, 60, True),
+                                              (150000, 24, False)])
+def test_one_long_row_among_many_short(orc, M, longest, binned):
+    # From 150,000 rows on, rows far past the mean (32 times its products) take
+    # the whole product to the bounds and the bins.
+    rng = np.random.default_rng(longest)
+    n = rng.integers(1, 4, M)
+    n[M // 3] = longest
+    A, B = _rows(rng, M, 5000, n), _between(rng, 5000, 5000, 2, 8)
+    for ops in ([A, B], [A, B, _between(rng, 5000, 3000, 1, 3)]):
+        for fl, labels in _labels(orc, ops).items():
+            assert any(x.endswith(".bounds") for x in labels) == binned, (fl, labels)

@@ -626,7 +626,7 @@ __device__ __forceinline__ void replay_direct(const DirectRowArgs& a, const RowP
             a.P.rp, a.P.ci, pv, sx, sh2);
         if (mask) {
             replay_write<MODE, TO>(mask, st[1], sx, sh2, p, book, row);
-            if (MODE == kSymb && p.row_cnt1 && lane < 2 && (mask >> lane & 1))
+            if (MODE != kNumExact && p.row_cnt1 && lane < 2 && (mask >> lane & 1))
                 p.row_cnt1[row + lane] = st[0].ns;
         }
         return mask;

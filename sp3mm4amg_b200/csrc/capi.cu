@@ -583,12 +583,14 @@ struct TailReads {
     long long total;   // nnz(C)
     int max_row;       // longest C row
     int retry;         // rows left for the retry launch
+    int left;          // rows the replayed kernel left
     unsigned err;      // device error word
 };
 
 // Scan row counts into row_ptr (allocated on first use) and read back, in
 // one round trip through the context's pinned words, the total, the longest
-// row, the retry count (d_retry, may be null) and the error word.
+// row, the retry and left counts (d_retry: the first, may be null: 0) and the
+// error word.
 int scan_read(sp3mm_ctx* ctx, int M, const int* row_cnt, DevBuf& rp, const int* d_retry,
               TailReads* out) {
     const cudaStream_t st = ctx->stream;
@@ -604,18 +606,19 @@ int scan_read(sp3mm_ctx* ctx, int M, const int* row_cnt, DevBuf& rp, const int* 
     CK(ctx, cudaMemsetAsync(sum, 0, sizeof(unsigned long long), st));
     launch_count_max(M, row_cnt, nullptr, mr, st, sum);
     unsigned* box = ctx->host_box;
-    box[2] = 0;
+    box[2] = box[3] = 0;
     CK(ctx, cudaMemcpyAsync(box, rp.as<int>() + M, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     if (d_retry)
-        CK(ctx, cudaMemcpyAsync(box + 2, d_retry, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(ctx, cudaMemcpyAsync(box + 3, ctx->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        CK(ctx, cudaMemcpyAsync(box + 2, d_retry, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(ctx, cudaMemcpyAsync(box + 6, ctx->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     CK(ctx, cudaMemcpyAsync(box + 4, sum, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                             st));
     CK(ctx, cudaStreamSynchronize(st));
     out->total = static_cast<long long>(*reinterpret_cast<unsigned long long*>(box + 4));
     out->max_row = static_cast<int>(box[1]);
     out->retry = static_cast<int>(box[2]);
-    out->err = box[3];
+    out->left = static_cast<int>(box[3]);
+    out->err = box[6];
     return SP3MM_OK;
 }
 
@@ -803,8 +806,8 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
     const bool tiny = !rr.direct && caps.np1 <= kTinyProducts;
     const bool replay = !tiny && M >= kReplayMinRows && caps.np1 >= kReplayMinProducts;
     DevBuf left;
-    if (replay) TRY(left.alloc(ctx, sizeof(int) * (static_cast<size_t>(M) + 1)));
-    int* n_left = left.as<int>() + M;
+    if (replay) TRY(left.alloc(ctx, sizeof(int) * static_cast<size_t>(M)));
+    int* n_left = &dc->left_count;
     auto geometry = [&](int mode) {
         RowGeom geo{};
         geo.block = 32 * kReplayWarps;
@@ -870,16 +873,13 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
             p.row_cnt1 = row_cnt1.as<int>();
         }
         TRY(rows(kSymb));
-        if (replay)
-            CK(ctx, cudaMemcpyAsync(ctx->host_box + 6, n_left, sizeof(int), cudaMemcpyDeviceToHost,
-                                    st));
         TRY(scan_read(ctx, M, row_cnt.as<int>(), rp, &dc->retry_count, &tr));
         if (tr.err) return check_device_err(ctx);
         // Where many rows outgrew the tables of the bound, the numeric pass
         // would run them on the retry kernel (about 13 us a thousand rows):
         // the rows are binned by their counts instead, unless most of them are
         // replayed.
-        const long long left = replay ? static_cast<int>(ctx->host_box[6]) : M;
+        const long long left = replay ? tr.left : M;
         rebin = !tiny && tr.retry > kRebinRetries + M / 256 && 2 * left > M;
         if (tr.retry > 0) {
             TRY(rr.run_retry(p, tr.retry, retry, s1_max, s2_max));

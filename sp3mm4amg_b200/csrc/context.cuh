@@ -161,6 +161,7 @@ struct Counters {
     int cursors[kLevels];
     int nmax;
     int retry_count;
+    int left_count;             // rows the replayed kernel left (read with retry_count)
     unsigned long long total;
     unsigned long long cursor;
 };

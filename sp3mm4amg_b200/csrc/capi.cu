@@ -968,13 +968,21 @@ int product_bounded(sp3mm_ctx* ctx, RowRunner& rr, int M, int N, int flavour, in
 }
 
 // ---------------------------------------------------------------------------
+// Products size launches by the longest rows that their operands record.  The
+// kernels flag a row past them and take nothing out of range; such a product is
+// formed again without the records (a caller's own sp3mm_dcsr may understate
+// them), and an error that is not theirs comes back.
+sp3mm_dcsr unrecorded(sp3mm_dcsr m) {
+    m.max_row = -1;
+    return m;
+}
+bool past_records(int rc, const sp3mm_dcsr& a, const sp3mm_dcsr& b) {
+    return (rc == SP3MM_EINVAL || rc == SP3MM_EDEVICE) && (a.max_row >= 0 || b.max_row >= 0);
+}
+
 // C = A*B.
-int spmm_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flavour, int out_vt,
-              sp3mm_dcsr* C) {
-    if (A.N != B.M)
-        return set_error(ctx, SP3MM_EINVAL, "inner dimensions differ (%d vs %d)", A.N, B.M);
-    if (A.val_type != B.val_type)
-        return set_error(ctx, SP3MM_EINVAL, "operands must share one value storage type");
+int spmm_recorded(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flavour,
+                  int out_vt, sp3mm_dcsr* C) {
     const int M = A.M;
     const cudaStream_t st = ctx->stream;
     int G = pick_group(ctx, B.M ? static_cast<double>(B.nnz) / B.M : 1.0);
@@ -1002,14 +1010,20 @@ int spmm_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flav
     RowRunner rr{ctx, false, kSymb, {}, PairRowArgs{view(A), view(B)}, -1, B.max_row};
     return product_rows(ctx, rr, M, B.N, flavour, out_vt, need, dc, G, d1, 0, B.N, 0, 0.0, C);
 }
+int spmm_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& A, const sp3mm_dcsr& B, int flavour, int out_vt,
+              sp3mm_dcsr* C) {
+    if (A.N != B.M)
+        return set_error(ctx, SP3MM_EINVAL, "inner dimensions differ (%d vs %d)", A.N, B.M);
+    if (A.val_type != B.val_type)
+        return set_error(ctx, SP3MM_EINVAL, "operands must share one value storage type");
+    const int rc = spmm_recorded(ctx, A, B, flavour, out_vt, C);
+    if (!past_records(rc, A, B)) return rc;
+    return spmm_recorded(ctx, unrecorded(A), unrecorded(B), flavour, out_vt, C);
+}
 
 // C = R*A*P, direct (row forwarding).
-int direct_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const sp3mm_dcsr& P,
-                int flavour, int out_vt, bool smoothed, sp3mm_dcsr* C) {
-    if (R.N != A.M || A.N != P.M)
-        return set_error(ctx, SP3MM_EINVAL, "inner dimensions differ");
-    if (R.val_type != A.val_type || A.val_type != P.val_type)
-        return set_error(ctx, SP3MM_EINVAL, "operands must share one value storage type");
+int direct_recorded(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A,
+                    const sp3mm_dcsr& P, int flavour, int out_vt, bool smoothed, sp3mm_dcsr* C) {
     const int M = R.M;
     const cudaStream_t st = ctx->stream;
     const double mean = std::max(A.M ? static_cast<double>(A.nnz) / A.M : 1.0,
@@ -1044,6 +1058,16 @@ int direct_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const 
                      smoothed};
     return product_rows(ctx, rr, M, P.N, flavour, out_vt, need, dc, G, d1, d2, A.N, P.N,
                         static_cast<double>(pmax), C, need_opt.as<int>());
+}
+int direct_impl(sp3mm_ctx* ctx, const sp3mm_dcsr& R, const sp3mm_dcsr& A, const sp3mm_dcsr& P,
+                int flavour, int out_vt, bool smoothed, sp3mm_dcsr* C) {
+    if (R.N != A.M || A.N != P.M)
+        return set_error(ctx, SP3MM_EINVAL, "inner dimensions differ");
+    if (R.val_type != A.val_type || A.val_type != P.val_type)
+        return set_error(ctx, SP3MM_EINVAL, "operands must share one value storage type");
+    const int rc = direct_recorded(ctx, R, A, P, flavour, out_vt, smoothed, C);
+    if (!past_records(rc, R, R)) return rc;
+    return direct_recorded(ctx, unrecorded(R), A, P, flavour, out_vt, smoothed, C);
 }
 
 void free_dcsr_arrays(sp3mm_ctx* ctx, sp3mm_dcsr* m) {
@@ -1924,7 +1948,12 @@ int sp3mm_spmm_rowsizes(sp3mm_ctx* ctx, const sp3mm_dcsr* A, const sp3mm_dcsr* B
     DevBuf rp;
     long long nnz = 0;
     TRY(scan_counts(ctx, M, row_cnt.as<int>(), rp, &nnz));
-    TRY(check_device_err(ctx));
+    const int rc = check_device_err(ctx);
+    if (past_records(rc, *B, *B)) {
+        const sp3mm_dcsr all = unrecorded(*B);
+        return sp3mm_spmm_rowsizes(ctx, A, &all, exact, rows_dev, total);
+    }
+    TRY(rc);
     if (rows_dev)
         CK(ctx, cudaMemcpyAsync(rows_dev, row_cnt.p, sizeof(int) * M, cudaMemcpyDeviceToDevice, st));
     CK(ctx, cudaStreamSynchronize(st));

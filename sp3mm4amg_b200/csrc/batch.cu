@@ -40,16 +40,13 @@ namespace {
 
 // need[g] = distinct-key bound of the first table of global row g (the
 // product count of its row of X*Y, at most Y.N); row_item[g] = its product.
-// *total += the output-size bound of every row (SpMM: need; direct:
-// min(R*A products times Z's longest row, Z.N)).  need_opt[g] = the
-// optimistic first-table size: need >> d1 capped at 8 sqrt(products) (long
-// rows repeat their columns; the single-product bound kernel uses the same
-// guess), or need itself when the row's products reach Y's column count
-// (such rows are dense).
+// need_opt[g] = the optimistic first-table size: need >> d1 capped at
+// 8 sqrt(products) (long rows repeat their columns; the single-product bound
+// kernel uses the same guess), or need itself when the row's products reach
+// Y's column count (such rows are dense).
 __global__ void k_batch_bounds(const BItem* __restrict__ items, const long long* __restrict__ bases,
                                int n, long long rows, int d1, int* need, int* need_opt,
-                               int* row_item, unsigned long long* total) {
-    unsigned long long ub = 0;
+                               int* row_item) {
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < rows;
          g += (long long)gridDim.x * blockDim.x) {
         int lo = 0, hi = n;   // largest b with bases[b] <= g; bases[n] = rows
@@ -80,17 +77,7 @@ __global__ void k_batch_bounds(const BItem* __restrict__ items, const long long*
         o = o > 64 ? o : (nd < 64 ? nd : 64);
         need_opt[g] = nd == 0 ? 0 : (u >= I->Y.N ? nd : max(1, static_cast<int>(o)));
         row_item[g] = lo;
-        if (I->kind == kBatchDirect) {
-            const long long zm = I->zmax >= 0 ? I->zmax : I->Z.N;
-            const long long b2 = u * zm;
-            ub += static_cast<unsigned long long>(b2 < I->Z.N ? b2 : I->Z.N);
-        } else {
-            ub += static_cast<unsigned long long>(u < I->Y.N ? u : I->Y.N);
-        }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ub += __shfl_xor_sync(0xffffffffu, ub, o);
-    if ((threadIdx.x & 31) == 0 && ub) atomicAdd(total, ub);
 }
 
 // Per-product output offset and length from the global row pointers.
@@ -701,8 +688,7 @@ int batch_plan(sp3mm_batch* b) {
         prof(ctx, "batch.bounds", [&] {
             k_batch_bounds<<<grid_for_rows(rows), 256, 0, st>>>(
                 b->d_items.as<BItem>(), b->d_bases.as<long long>(), n, rows, b->d1,
-                b->d_need.as<int>(), b->d_need_opt.as<int>(), b->d_row_item.as<int>(),
-                &dc->total);
+                b->d_need.as<int>(), b->d_need_opt.as<int>(), b->d_row_item.as<int>());
         });
         note_launch();
         CK(ctx, cudaGetLastError());
@@ -739,12 +725,20 @@ int batch_plan(sp3mm_batch* b) {
         // and their A*P0 steps write well under their operands' nonzeros;
         // reserving more made the pool map tens of GB for a batch of large
         // hierarchies' first levels.
+        // (Small batches book what their results can hold at most.)
         const size_t eb = sizeof(int) + vbytes(b->to);
         long long in_nnz = 0;
-        for (const BItem& I : b->items)
-            in_nnz += I.X.nnz + I.Y.nnz + (I.kind == kBatchDirect ? I.Z.nnz : 0);
-        unsigned long long cap = std::max<unsigned long long>(1ULL << 20, 2ULL * in_nnz) +
-                                 b->chunks.size() * kReplayWarps * kReplayBook;
+        double most = 0.0;
+        for (const BItem& I : b->items) {
+            const bool direct = I.kind == kBatchDirect;
+            in_nnz += I.X.nnz + I.Y.nnz + (direct ? I.Z.nnz : 0);
+            double m = static_cast<double>(I.X.nnz) * (I.ymax >= 0 ? I.ymax : I.Y.N);
+            if (direct) m *= I.zmax >= 0 ? I.zmax : I.Z.N;
+            most += std::min(m, static_cast<double>(I.M) * I.N);
+        }
+        unsigned long long cap = std::max<unsigned long long>(1ULL << 20, 2ULL * in_nnz);
+        if (most < static_cast<double>(cap)) cap = static_cast<unsigned long long>(most);
+        cap += b->chunks.size() * kReplayWarps * kReplayBook;
         if (cap * eb > (size_t(1) << 30) && pool_idle_bytes(ctx) < cap * eb)
             cap = std::min<unsigned long long>(
                 cap, std::max<unsigned long long>(1ULL << 20, free_device_bytes(ctx) / 2 / eb));

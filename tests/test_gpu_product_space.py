@@ -212,3 +212,26 @@ def test_space_of_uneven_rows(variant):
         got[0].free()
         for m in d:
             m.free()
+
+
+def test_space_of_a_small_batch(orc):
+    # A batch books no more than its results can hold: here 2 MB at most, not
+    # the 12 MB of the least that larger batches take.
+    from sp3mm4amg_b200 import problems as pb
+    p = pb.stencil_problem(2, (50, 60))
+    ops = (p.R, p.A, p.P)
+    with S.Context() as ctx:
+        d = [ctx.upload(m) for m in ops]
+        got = []
+
+        def run():
+            got.append(ctx.batch([tuple(d), (d[0], d[1])]))
+            got[0].run()
+        peak = _pool_peak(ctx, run)
+        assert peak < 6 << 20, peak
+        for i, want in enumerate((orc.sp3mm_direct(*ops), orc.spmm(*ops[:2]))):
+            cmp = O.compare(got[0].result(i).download(), want, rtol=0.0)
+            assert cmp["ok"] and cmp["bitwise_equal"] == want.nnz, (i, cmp)
+        got[0].free()
+        for m in d:
+            m.free()

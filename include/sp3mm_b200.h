@@ -250,7 +250,9 @@ typedef struct {
     int32_t *col;
     void *val;
     int32_t val_type;   /* SP3MM_F64 or SP3MM_F32 */
-    int32_t max_row;    /* longest row, or -1 when unknown */
+    int32_t max_row;    /* longest row, or -1 when unknown: products size their
+                         * launches by it.  One that is too small costs a second
+                         * try (SP3MM_EINVAL for A or P of a direct product). */
 } sp3mm_dcsr;
 
 typedef struct sp3mm_ctx sp3mm_ctx;

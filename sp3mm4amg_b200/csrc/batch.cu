@@ -429,9 +429,10 @@ int join_replay(sp3mm_batch* b, int mode) {
 }
 
 // The direct products whose rows the replayed kernel may take, cut into runs
-// of rows for one wave of CTAs: X's longest row (where it is not known, its
-// mean) times Y's longest within kBoundedProducts, in two classes by the
-// kernel's unroll.  Rows past the capacities stay with the tiers.  20 grids of
+// of rows for one wave of CTAs: X's longest row (where it is not known, a
+// quarter above its mean and two) times Y's longest within kBoundedProducts, in
+// two classes by the kernel's unroll.  Rows past the capacities stay with the
+// tiers.  20 grids of
 // 1e3 to 2e5 points: replayed numeric pass 0.73 -> 0.51 ms; booked plan 0.52 ->
 // 0.41 ms of kernels (one class for both sizes of rows: 0.47).
 int plan_replay(sp3mm_batch* b) {

@@ -487,13 +487,8 @@ bool plain_tuning(const sp3mm_ctx* ctx) {
     return ctx->tune_G == 0 && ctx->tune_d1 < 0 && ctx->tune_d2 < 0;
 }
 
-// Products whose longest rows bound every row's products by kBoundedProducts
-// need no bounds pass and no binning: the bound sizes one launch over all
-// rows (a bounds launch, two binning launches and a host round trip fewer:
-// the 64x64 product 106 -> 85 us).
-
 // Symbolic retries (and M / 256 of them, what binning M rows takes) from which
-// the exact numeric pass of such a product bins its rows: 300,000 rows of 3 to
+// the exact numeric pass of a bounded product bins its rows: 300,000 rows of 3 to
 // 6 times 5 to 15 random entries, all but a few retried, 6.1 -> 4.3 ms.
 constexpr int kRebinRetries = 4096;
 
@@ -501,8 +496,12 @@ constexpr int kRebinRetries = 4096;
 constexpr int kUnevenMinRows = 150000;
 constexpr double kUnevenRatio = 32.0;
 
-// Whether rows of at most k1 steps of l1 products (and, direct, of P rows of
-// at most l2) are bounded so, and the replayed kernel's capacities.
+// Products whose longest rows bound every row's products by kBoundedProducts
+// need no bounds pass and no binning: the bound sizes one launch over all
+// rows (a bounds launch, two binning launches and a host round trip fewer:
+// the 64x64 product 106 -> 85 us).  Whether rows of at most k1 steps of l1
+// products (and, direct, of P rows of at most l2) are bounded so, and the
+// replayed kernel's capacities.
 bool bounded_rows(bool direct, int k1, int l1, int n1, int l2, int n2, ReplayCaps* c) {
     if (k1 < 0 || l1 < 0 || l2 < 0 || k1 > kReplayMaxColumns) return false;
     const long long np = static_cast<long long>(k1) * l1;

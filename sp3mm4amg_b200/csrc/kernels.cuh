@@ -121,8 +121,9 @@ size_t lanes_row_bytes(int mode, int S1, int S2);
 cudaError_t launch_pair_lanes(const PairRowArgs& a, const RowParams& p, int mode,
                               const RowGeom& geo, cudaStream_t st);
 size_t pair_lanes_row_bytes(int mode, int S);
-// Rows of few products (rowreplay.cuh), one warp per row, consecutive rows
-// per warp.  replay_bytes: shared memory per warp.
+// Rows of few products (rowreplay.cuh): a run of consecutive rows per CTA, two
+// at a time per warp, pairs dealt out to the warps in turn.  replay_bytes:
+// shared memory of a CTA of `warps` warps.
 cudaError_t launch_direct_replay(const DirectRowArgs& a, const RowParams& p, int mode,
                                  const RowGeom& geo, cudaStream_t st);
 cudaError_t launch_pair_replay(const PairRowArgs& a, const RowParams& p, int mode,

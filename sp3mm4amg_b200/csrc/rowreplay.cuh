@@ -2,17 +2,17 @@
 // from one worked-out pattern (sm_100a).
 //
 // A row's sums are fixed by which of its products meet in a column.  A CTA
-// takes a run of consecutive rows and works that out once, for the row in
-// the middle of its run: per stage, the template holds the products in the
-// reference's order -- left position t ascending, then the selected right
-// row's entries ascending (code/src/include/SpMMUtilsGeneric.h:39-55) -- with
-// their columns and, per distinct column, the list of its products in that
-// order.  Another row whose right rows have the same lengths and whose
-// product columns are the template's plus one constant meets in the same
-// places, whatever its values: that is checked, product by product, as the
-// products are loaded.  On the inside of a structured grid nearly every row
-// passes; the others go to a list that the register-product kernels run
-// (rowlanes.cuh).
+// takes a run of consecutive rows and works that out once, for a row of the
+// most frequent length among 32 spread over its run (replay_pick): per stage,
+// the template holds the products in the reference's order -- left position t
+// ascending, then the selected right row's entries ascending
+// (code/src/include/SpMMUtilsGeneric.h:39-55) -- with their columns and, per
+// distinct column, the list of its products in that order.  Another row whose
+// right rows have the same lengths and whose product columns are the
+// template's plus one constant meets in the same places, whatever its values:
+// that is checked, product by product, as the products are loaded.  On the
+// inside of a structured grid nearly every row passes; the others go to a list
+// that the register-product kernels run (rowlanes.cuh).
 //
 // The sums then need no table: each lane owns a column and adds its listed
 // products one after another, from 0.0, in the reference's order, so values

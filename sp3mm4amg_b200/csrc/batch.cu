@@ -628,24 +628,20 @@ int ensure_numeric(sp3mm_batch* b) {
                                 ctx->stream);
     // Replaying pays where most rows match: on irregular patterns its CTAs only
     // held the tiers up (5 products of 3,000 to 40,000 random rows: 0.80 ms a pass against 0.64).
-    const unsigned* kept = ctx->host_box + 8;
     if (M > 0 && !b->replays.empty()) {
-        int* d_kept = reinterpret_cast<int*>(b->d_counters.as<Counters>() + 2) + 2;
         const int second = b->replays.size() > 1 ? b->replays[1].first : INT_MAX;
-        CK(ctx, cudaMemsetAsync(d_kept, 0, 2 * sizeof(int), ctx->stream));
         k_batch_keep_chunks<<<static_cast<int>(b->chunks.size()), 128, 0, ctx->stream>>>(
             b->d_items.as<BItem>(), b->d_chunks.as<int4>(), second,
-            b->d_done.as<unsigned char>(), d_kept);
+            b->d_done.as<unsigned char>(), dc->kept);
         note_launch();
-        CK(ctx, cudaMemcpyAsync(ctx->host_box + 8, d_kept, 2 * sizeof(int),
-                                cudaMemcpyDeviceToHost, ctx->stream));
         k_batch_drop_done<<<grid_for_rows(M), 256, 0, ctx->stream>>>(
             M, b->d_done.as<unsigned char>(), b->d_need.as<int>());
         note_launch();
         CK(ctx, cudaGetLastError());
     }
-    TRY(bin_rows(ctx, M, b->d_need.as<int>(), 0, 32, dc, nullptr, b->nbins));   // (synchronises)
-    for (size_t k = 0; M > 0 && k < b->replays.size(); ++k) b->replays[k].numeric = kept[k] > 0;
+    TRY(bin_rows(ctx, M, b->d_need.as<int>(), 0, 32, dc, nullptr, b->nbins));
+    for (size_t k = 0; M > 0 && k < b->replays.size(); ++k)
+        b->replays[k].numeric = b->nbins.kept[k] > 0;
     ProfSpan span(ctx, "batch.graph");
     return build_numeric(b);
 }
@@ -681,7 +677,7 @@ int batch_plan(sp3mm_batch* b) {
     const size_t cbytes = sizeof(Counters) * 2 + 4 * sizeof(int);
     TRY(b->d_counters.alloc(ctx, cbytes));
     Counters* dc = b->d_counters.as<Counters>();
-    int* rinfo = reinterpret_cast<int*>(dc + 2);   // retry count, retry need (2: kept chunks)
+    int* rinfo = reinterpret_cast<int*>(dc + 2);   // retry count, retry need
     CK(ctx, cudaMemsetAsync(b->d_cnt1.p, 0, sizeof(int) * R1, st));
     CK(ctx, cudaMemsetAsync(b->d_cnt2.p, 0, sizeof(int) * R1, st));
     CK(ctx, cudaMemsetAsync(b->d_counters.p, 0, cbytes, st));

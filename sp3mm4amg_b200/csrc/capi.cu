@@ -166,6 +166,8 @@ int bin_rows(sp3mm_ctx* ctx, int M, const int* need, int shift, int G, Counters*
     }
     b.counts[kLevels] = h.counts[kLevels];
     b.nmax = h.nmax;
+    b.kept[0] = h.kept[0];
+    b.kept[1] = h.kept[1];
     b.total = h.total;
     CK(ctx, cudaMemcpyAsync(dcnt->cursors, h.cursors, sizeof h.cursors, cudaMemcpyHostToDevice,
                             ctx->stream));

@@ -162,6 +162,7 @@ struct Counters {
     int nmax;
     int retry_count;
     int left_count;             // rows the replayed kernel left (read with retry_count)
+    int kept[2];                // a batch's runs of rows that it replays, by class
     unsigned long long total;
     unsigned long long cursor;
 };
@@ -171,6 +172,7 @@ struct Bins {
     int counts[kLevels + 1] = {};
     int offsets[kLevels] = {};
     int nmax = 0;
+    int kept[2] = {};
     unsigned long long total = 0;
     DevBuf level, lists;
 };

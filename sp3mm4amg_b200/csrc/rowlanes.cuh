@@ -196,8 +196,12 @@ __host__ __device__ __forceinline__ size_t wlanes_bytes(bool num, int S1, int S2
     return static_cast<size_t>(S1 + S2) * (num ? 16 : 8);
 }
 
+// (The packed symbolic pass fits five CTAs of registers per SM, 48 a thread; two
+// more, which the choice of list or all rows took, left four: 60,000-point kNN
+// product of 8 neighbours, symbolic kernels 114 -> 128 us.)
 template <int MODE, typename TV, typename TO, bool PACK>
-__global__ void __launch_bounds__(256, 4) k_direct_lanes(DirectRowArgs a, RowParams p) {
+__global__ void __launch_bounds__(256, MODE == kSymb && PACK ? 5 : 4)
+    k_direct_lanes(DirectRowArgs a, RowParams p) {
     constexpr bool NUM = MODE != kSymb;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;

@@ -248,6 +248,11 @@ constexpr int kBatchDenseMinSlots = 2048;
 // columns per row, within the CTA's 4096-entry list.
 constexpr int kBatchDenseMaxSlots = 4096;
 
+// Rows of at most 32 << kOneTierLevel slots that make one tier when they are at
+// most kOneTierRows.
+constexpr int kOneTierLevel = 2;
+constexpr long long kOneTierRows = 4096;
+
 // Tiers over the non-empty levels of `bins`.  A tier's tables hold
 // 32 << (its top level + extra) slots per warp (extra: the numeric slack,
 // or the symbolic shift d1 so that a proven-size retry still fits).  Tiers
@@ -269,8 +274,14 @@ int make_tiers(sp3mm_batch* b, const Bins& bins, int mode, int extra, int tv, in
     bool all_direct = !b->items.empty();
     for (const BItem& I : b->items) all_direct = all_direct && I.kind == kBatchDirect;
     const bool dense_ok = all_direct && batch_dense_smem() + 1024 <= ctx->smem_optin;
+    // Few small rows take one launch in a plan's pass, with the tables of the
+    // largest: the branch streams of more cost 8 grids of 500 to 700 points 10 of
+    // 200 us.
+    long long small = 0;
+    for (int L = 0; L <= kOneTierLevel; ++L) small += bins.counts[L];
+    const int one = mode != kNumExact && small <= kOneTierRows ? kOneTierLevel : 0;
     auto tier_of = [&](int L) {
-        if (b->auto_split) return L;
+        if (b->auto_split) return std::max(L, one);
         int t = 0;
         for (int s : b->splits)
             if (L >= s) ++t;

@@ -77,3 +77,26 @@ def test_rows_replayed_in_the_numeric_pass(orc, which, fl):
         for x in d:
             for m in x:
                 m.free()
+
+
+@pytest.mark.parametrize("fl", [S.UB, S.SYMBNUM])
+@pytest.mark.parametrize("rows", [4096, 4097])
+def test_small_rows_in_one_tier(orc, rows, fl):
+    # Rows of 0 to 100 products on both sides of the count up to which the
+    # plan's pass gives them one launch, with heavier rows beside them.
+    rng = np.random.default_rng(rows)
+    A, P = _random(rng, 500, 700, 1, 10), _random(rng, 700, 300, 1, 3)
+    ops = [[_random(rng, rows - 300, 500, 0, 10), A, P], [_random(rng, 300, 500, 1, 3), A, P],
+           [_random(rng, 200, 500, 60, 90), A, P]]
+    pair = (ops[0][0], A)
+    with S.Context() as ctx:
+        d = [[ctx.upload(m) for m in o] for o in ops + [list(pair)]]
+        b = ctx.batch([tuple(x) for x in d], S.F64, fl)
+        b.run()
+        for i, want in enumerate([orc.sp3mm_direct(*o) for o in ops] + [orc.spmm(*pair)]):
+            cmp = O.compare(b.result(i).download(), want, rtol=0.0)
+            assert cmp["ok"] and cmp["bitwise_equal"] == want.nnz, (i, cmp)
+        b.free()
+        for x in d:
+            for m in x:
+                m.free()

@@ -43,7 +43,8 @@ constexpr int kReplayBook = 512;
 // kReplayMinProducts try the replayed rows.  Below that many rows the
 // templates serve too few (direct, 7-point box: 6,840 rows 87 us against 57
 // on the lanes kernel alone, 21,000 rows 126 against 127, 262,144 rows 0.95 ms
-// against 1.51); with fewer products a row is one batch of the lanes kernel,
+// against 1.51; where nothing matches, the try costs 39 of 540 us at 20,000
+// random rows, 44 us of 5 ms at 300,000); with fewer products a row is one batch of the lanes kernel,
 // and the rows of A*P alternate between patterns.
 constexpr int kReplayMinRows = 16384;
 constexpr int kReplayMinProducts = 48;

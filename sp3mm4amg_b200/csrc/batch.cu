@@ -134,11 +134,12 @@ __global__ void k_batch_drop_done(long long rows, const unsigned char* __restric
 }
 
 // Chunks of the replayed kernel (one per CTA, `second` on of the second class)
-// of whose rows the plan's pass replayed less than 1 in kKeepChunk leave them
-// all to the tiers: their flags are cleared and their runs emptied.  *kept (of
-// the class) counts the others.  (Less than half: a pass over 20 grids of 1,000
-// to 200,000 points 0.56 ms instead of 0.53.)
-constexpr int kKeepChunk = 8;
+// of whose rows the plan's pass replayed less than 1 in kKeepChunk, or just the
+// template's pair, leave them all to the tiers: their flags are cleared and
+// their runs emptied.  *kept (of the class) counts the others.  A pass over 20
+// grids of 1,000 to 200,000 points, whose edge runs match in part, in us by
+// kKeepChunk: 2 547, 8 523, 16 515, 32 514; 514 with all runs kept.
+constexpr int kKeepChunk = 32;
 __global__ void __launch_bounds__(128) k_batch_keep_chunks(const BItem* __restrict__ items,
                                                            int4* chunks, int second,
                                                            unsigned char* done, int* kept) {
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(128) k_batch_keep_chunks(const BItem* __restri
         const int r = r0 + threadIdx.x;
         n += __syncthreads_count(r < ch.z && d[r]);
     }
-    if (kKeepChunk * n < ch.z - ch.y || n == 0) {
+    if (kKeepChunk * n < ch.z - ch.y || n <= 2) {
         for (int r = ch.y + threadIdx.x; r < ch.z; r += blockDim.x) d[r] = 0;
         if (threadIdx.x == 0) chunks[blockIdx.x].z = ch.y;
     } else if (threadIdx.x == 0) {

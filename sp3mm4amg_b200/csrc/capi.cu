@@ -1987,7 +1987,7 @@ int sp3mm_transpose(sp3mm_ctx* ctx, const sp3mm_dcsr* A, sp3mm_dcsr* AT) {
     launch_count_max(M, counts, nullptr, mr, st);
     launch_transpose_scatter(view(*A), rp.as<int>(), counts + words, ci.as<int>(), v.p, st);
     launch_sort_rows(M, rp.as<int>(), ci.as<int>(), v.p, A->val_type, static_cast<int>(A->nnz), st,
-                     ctx->d_err);
+                     ctx->d_err, mr);
     CK(ctx, cudaGetLastError());
     unsigned* box = ctx->host_box;
     CK(ctx, cudaMemcpyAsync(box, mr, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -458,10 +458,12 @@ __device__ __forceinline__ void sort_row_ranks(int* sk, double* sv, int b, int n
 template <bool NET>
 __global__ void __launch_bounds__(kSortThreads) k_sort_rows_cta(int M, int chunk, const int* rp,
                                                                 int* ci, void* v, int vt,
-                                                                unsigned* err) {
+                                                                unsigned* err,
+                                                                const int* longest) {
     constexpr int kMin = NET ? kSortRankRow : 32, kMax = NET ? kSortSmemRow : kSortRankRow;
     __shared__ __align__(16) int sk[NET ? 4 : kMax + 4];
     __shared__ std::conditional_t<NET, unsigned long long, double> sv[kMax];
+    if (NET && longest && *longest <= kMin) return;
     const int lane = threadIdx.x & 31;
     for (long long r0 = blockIdx.x * static_cast<long long>(chunk); r0 < M;
          r0 += gridDim.x * static_cast<long long>(chunk)) {
@@ -704,7 +706,7 @@ void launch_transpose_scatter(const CsrView& A, const int* t_rp, int* cursor, in
 }
 
 void launch_sort_rows(int M, const int* rp, int* ci, void* v, int vt, int max_row,
-                      cudaStream_t st, unsigned* err) {
+                      cudaStream_t st, unsigned* err, const int* longest) {
     if (M == 0 || max_row <= 1) return;
     k_sort_rows<<<grid_for(static_cast<long long>(M) * 32, 256), 256, 0, st>>>(M, rp, ci, v, vt,
                                                                               err);
@@ -714,10 +716,12 @@ void launch_sort_rows(int M, const int* rp, int* ci, void* v, int vt, int max_ro
         const int ctas = 148 * 8;
         const int chunk = M < ctas ? 1 : M / ctas < 32 ? M / ctas : 32;
         const int grid = grid_for(M, chunk, ctas);
-        k_sort_rows_cta<false><<<grid, kSortThreads, 0, st>>>(M, chunk, rp, ci, v, vt, err);
+        k_sort_rows_cta<false><<<grid, kSortThreads, 0, st>>>(M, chunk, rp, ci, v, vt, err,
+                                                              nullptr);
         note_launch();
         if (max_row > kSortRankRow) {
-            k_sort_rows_cta<true><<<grid, kSortThreads, 0, st>>>(M, chunk, rp, ci, v, vt, err);
+            k_sort_rows_cta<true><<<grid, kSortThreads, 0, st>>>(M, chunk, rp, ci, v, vt, err,
+                                                                 longest);
             note_launch();
         }
     }

@@ -255,19 +255,20 @@ struct RowRunner {
     // R its transpose (a hierarchy's own level).
     bool smoothed = false;
 
-    // Entries of booking space (a product that overflows it is redone with
-    // exact sizes): results may hold several times their operands' nonzeros
-    // (A*A*A of a 7-point operator 3 times, R*A*P over a random graph 8), and
-    // eight times them costs nothing but the space.  A hierarchy's levels are
-    // the exception: for the first product of a 128^3 one that is 2.8 GB
-    // allocated and freed per build, and a program that holds its last
-    // hierarchy while it builds the next made the pool remap it: 30 ms a
-    // build, against 18.1-20.5 with the operands' nonzeros once, and 18.4
-    // without the held one.  Once is enough where the aggregates' points share
-    // neighbours, that is where P holds fewer entries than A: at most 3/4 of
-    // them on grids and narrow bands, whose products hold at most 0.47 of the
-    // operands' nonzeros; 0.96-1.0 on kNN and random graphs and wide bands,
-    // whose products hold 2.3 to 10.6 times.
+    // Entries of booking space (a product that overflows it is redone with exact
+    // sizes): results may hold several times their operands' nonzeros (A*A*A of a
+    // 7-point operator 3 times, R*A*P over a random graph 8), and eight times them
+    // costs little once the pool has grown to it (128^3 products whose last three
+    // results are held: 1.10 ms with eight times, 1.09 with once; the first dozens
+    // of calls 1.3-1.4 against 1.1).  A hierarchy's levels are the exception: for
+    // the first product of a 128^3 one that is 2.8 GB allocated and freed per
+    // build, and a program that holds its last hierarchy while it builds the next
+    // made the pool remap it: 30 ms a build, against 18.1-20.5 with the operands'
+    // nonzeros once, and 18.4 without the held one.  Once is enough where the
+    // aggregates' points share neighbours, that is where P holds fewer entries
+    // than A: at most 3/4 of them on grids and narrow bands, whose products hold
+    // at most 0.47 of the operands' nonzeros; 0.96-1.0 on kNN and random graphs
+    // and wide bands, whose products hold 2.3 to 10.6 times.
     unsigned long long booked_entries() const {
         if (!direct) return 8ULL * static_cast<unsigned long long>(pa.A.nnz + pa.B.nnz);
         const unsigned long long all =

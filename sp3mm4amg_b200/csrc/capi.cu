@@ -1987,12 +1987,19 @@ int sp3mm_transpose(sp3mm_ctx* ctx, const sp3mm_dcsr* A, sp3mm_dcsr* AT) {
     CK(ctx, cudaMemsetAsync(mr, 0, sizeof(int), st));
     launch_count_max(M, counts, nullptr, mr, st);
     launch_transpose_scatter(view(*A), rp.as<int>(), counts + words, ci.as<int>(), v.p, st);
-    launch_sort_rows(M, rp.as<int>(), ci.as<int>(), v.p, A->val_type, static_cast<int>(A->nnz), st,
-                     ctx->d_err, mr);
+    launch_sort_rows(M, rp.as<int>(), ci.as<int>(), v.p, A->val_type, kSortRankRow, st,
+                     ctx->d_err);
     CK(ctx, cudaGetLastError());
     unsigned* box = ctx->host_box;
     CK(ctx, cudaMemcpyAsync(box, mr, sizeof(int), cudaMemcpyDeviceToHost, st));
     TRY(check_device_err(ctx));   // synchronises: box is complete
+    // (a launch for the few transposes that have such rows: 3 us for each of a
+    // hierarchy's otherwise)
+    if (static_cast<int>(box[0]) > kSortRankRow) {
+        launch_sort_long_rows(M, rp.as<int>(), ci.as<int>(), v.p, A->val_type, st, ctx->d_err);
+        CK(ctx, cudaGetLastError());
+        TRY(check_device_err(ctx));
+    }
     AT->M = M;
     AT->N = A->M;
     AT->nnz = A->nnz;

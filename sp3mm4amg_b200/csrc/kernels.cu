@@ -367,11 +367,11 @@ __global__ void __launch_bounds__(256) k_transpose_scatter(CsrView A, int lg, co
 // warp per row with a bitonic network took 1.13 ms over the levels of a 128^3
 // hierarchy, this 0.43.  Ranks take n^2 comparisons: rows past kSortRankRow
 // entries go to a launch of their own (NET), a bitonic network of one size by
-// the CTA (transpose with 1,000 rows of 2,000: 1.28 -> 0.43 ms; both in one
+// the CTA (transpose with 1,000 rows of 2,000: 1.28 -> 0.46 ms; both in one
 // kernel made rows of 700 8 % slower).  A column met twice is flagged where err
 // is given.
 constexpr int kSortSmemRow = 2048;
-constexpr int kSortRankRow = kSortSmemRow / 2;
+static_assert(kSortRankRow == kSortSmemRow / 2, "the network's one size");
 constexpr int kSortThreads = 128;
 
 // Bitonic network over kSortSmemRow keys.
@@ -458,12 +458,10 @@ __device__ __forceinline__ void sort_row_ranks(int* sk, double* sv, int b, int n
 template <bool NET>
 __global__ void __launch_bounds__(kSortThreads) k_sort_rows_cta(int M, int chunk, const int* rp,
                                                                 int* ci, void* v, int vt,
-                                                                unsigned* err,
-                                                                const int* longest) {
+                                                                unsigned* err) {
     constexpr int kMin = NET ? kSortRankRow : 32, kMax = NET ? kSortSmemRow : kSortRankRow;
     __shared__ __align__(16) int sk[NET ? 4 : kMax + 4];
     __shared__ std::conditional_t<NET, unsigned long long, double> sv[kMax];
-    if (NET && longest && *longest <= kMin) return;
     const int lane = threadIdx.x & 31;
     for (long long r0 = blockIdx.x * static_cast<long long>(chunk); r0 < M;
          r0 += gridDim.x * static_cast<long long>(chunk)) {
@@ -705,26 +703,38 @@ void launch_transpose_scatter(const CsrView& A, const int* t_rp, int* cursor, in
     note_launch();
 }
 
+namespace {
+// CTAs of a row sort and the row lengths each looks up at once: few rows one by
+// one, many 32 at a time.
+struct SortGrid {
+    int grid, chunk;
+};
+SortGrid sort_grid(int M) {
+    const int ctas = 148 * 8;
+    const int chunk = M < ctas ? 1 : M / ctas < 32 ? M / ctas : 32;
+    return {grid_for(M, chunk, ctas), chunk};
+}
+}  // namespace
+
 void launch_sort_rows(int M, const int* rp, int* ci, void* v, int vt, int max_row,
-                      cudaStream_t st, unsigned* err, const int* longest) {
+                      cudaStream_t st, unsigned* err) {
     if (M == 0 || max_row <= 1) return;
     k_sort_rows<<<grid_for(static_cast<long long>(M) * 32, 256), 256, 0, st>>>(M, rp, ci, v, vt,
                                                                               err);
     note_launch();
     if (max_row > 32) {
-        // Few rows: one per CTA; many: 32 lengths looked up at once.
-        const int ctas = 148 * 8;
-        const int chunk = M < ctas ? 1 : M / ctas < 32 ? M / ctas : 32;
-        const int grid = grid_for(M, chunk, ctas);
-        k_sort_rows_cta<false><<<grid, kSortThreads, 0, st>>>(M, chunk, rp, ci, v, vt, err,
-                                                              nullptr);
+        const SortGrid g = sort_grid(M);
+        k_sort_rows_cta<false><<<g.grid, kSortThreads, 0, st>>>(M, g.chunk, rp, ci, v, vt, err);
         note_launch();
-        if (max_row > kSortRankRow) {
-            k_sort_rows_cta<true><<<grid, kSortThreads, 0, st>>>(M, chunk, rp, ci, v, vt, err,
-                                                                 longest);
-            note_launch();
-        }
     }
+    if (max_row > kSortRankRow) launch_sort_long_rows(M, rp, ci, v, vt, st, err);
+}
+
+void launch_sort_long_rows(int M, const int* rp, int* ci, void* v, int vt, cudaStream_t st,
+                           unsigned* err) {
+    const SortGrid g = sort_grid(M);
+    k_sort_rows_cta<true><<<g.grid, kSortThreads, 0, st>>>(M, g.chunk, rp, ci, v, vt, err);
+    note_launch();
 }
 
 void launch_colparts_ub(const CsrView& A, int gridCols, const long long* bColOffsets,

@@ -217,10 +217,14 @@ void launch_col_counts(long long nnz, const int* ci, int* counts, cudaStream_t s
 void launch_transpose_scatter(const CsrView& A, const int* t_rp, int* cursor, int* t_ci,
                               void* t_v, cudaStream_t st);
 // max_row: no row is longer (the sort kernels skip the rows they do not handle).
-// err (optional): flagged when a row holds a column twice.  longest (optional):
-// the longest row on the device, by which a launch for longer ones ends at once.
+// err (optional): flagged when a row holds a column twice.
 void launch_sort_rows(int M, const int* rp, int* ci, void* v, int vtype, int max_row,
-                      cudaStream_t st, unsigned* err = nullptr, const int* longest = nullptr);
+                      cudaStream_t st, unsigned* err = nullptr);
+// The launch of launch_sort_rows for rows of more than kSortRankRow entries
+// (those past 2,048 are its first launch's).
+constexpr int kSortRankRow = 1024;
+void launch_sort_long_rows(int M, const int* rp, int* ci, void* v, int vtype, cudaStream_t st,
+                           unsigned* err);
 
 // 2D column-partition upper bounds.
 void launch_colparts_ub(const CsrView& A, int gridCols, const long long* bColOffsets,
